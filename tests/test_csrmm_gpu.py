@@ -108,3 +108,41 @@ def test_csrmm_size_errors(ctrl):
     st = api.lib().clsparseDcsrmm(C.byref(api.scalar(one)), C.byref(A.s), C.byref(bad_ld), C.byref(api.scalar(one)),
                                   C.byref(good_c), ctrl.handle)
     assert st == L.clsparseInvalidSize
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
+@pytest.mark.parametrize("pad,off", [(0, 0), (2, 2), (1, 0), (0, 1), (4, 4)])
+@pytest.mark.parametrize("ncols", [2, 4, 6, 20, 40, 68, 129, 132, 260])
+def test_csrmm_vector_widths(ctrl, dtype, ncols, pad, off):
+    """Every vector width and lane split of the row-major path: column counts
+    around one vector, one tile (32 vectors) and several; rows of 0, 1 and
+    around 32 and 128 nonzeros; rows and bases that allow 16-byte, 8-byte or
+    only scalar access. Tolerance: the FP32 sums of at most 129 products and
+    the final combination stay within 130 roundings of the absolute sum; the
+    bars of the tests above are 16 times that for FP64 and 1.6 times for FP32."""
+    rng = np.random.default_rng(ncols + pad + off)
+    lens = [0, 1, 2, 3, 4, 5, 31, 32, 33, 64, 127, 128, 129, 0, 7, 7] * 5
+    n, m = len(lens), 300
+    rp, col, val = matgen.random_lengths(lens, m, seed=ncols)
+    A = api.CsrMatrix.from_numpy(rp, col, val, num_cols=m, dtype=dtype)
+    B, C0 = rng.uniform(-1, 1, (m, ncols)), rng.uniform(-1, 1, (n, ncols))
+    ld = ncols + pad
+    fill = torch.full((off,), float("nan"), dtype=dtype, device="cuda")
+    tb = torch.cat([fill, layout(B, ld, L.rowMajor, dtype)])
+    tc = torch.cat([fill, layout(C0, ld, L.rowMajor, dtype)])
+    db, dc = dense(tb, m, ncols, ld, L.rowMajor), dense(tc, n, ncols, ld, L.rowMajor)
+    db.off_values = dc.off_values = off
+    a = torch.tensor([-0.75], dtype=dtype, device="cuda")
+    b = torch.tensor([0.5], dtype=dtype, device="cuda")
+    fn = api.lib().clsparseDcsrmm if dtype == torch.float64 else api.lib().clsparseScsrmm
+    assert fn(C.byref(api.scalar(a)), C.byref(A.s), C.byref(db), C.byref(api.scalar(b)), C.byref(dc), ctrl.handle) == 0
+    t = np.float64 if dtype == torch.float64 else np.float32
+    Am = sp.csr_matrix((np.asarray(val, t).astype(np.float64), col.astype(np.int64), rp.astype(np.int64)), shape=(n, m))
+    Bc, Cc = np.asarray(B, t).astype(np.float64), np.asarray(C0, t).astype(np.float64)
+    ref = -0.75 * (Am @ Bc) + 0.5 * Cc
+    scale = 0.75 * (abs(Am) @ abs(Bc)) + 0.5 * abs(Cc) + 1e-300
+    raw = tc.cpu().numpy().astype(np.float64)
+    assert off == 0 or np.isnan(raw[:off]).all()
+    out = raw[off:].reshape(n, ld)
+    assert np.max(np.abs(out[:, :ncols] - ref) / scale) <= TOL[dtype] * 10
+    np.testing.assert_array_equal(out[:, ncols:], 0)
