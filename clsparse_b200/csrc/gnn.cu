@@ -372,13 +372,60 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// grad[off + i] += sum over `ntiles` partial records (fixed order).
-__global__ void reduce_parts(const float* __restrict__ part, int rec, int ntiles, float* __restrict__ grad,
-                             int off_w, int off_b, int nw) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= rec) return;
+// grad[off + i] += sum over `ntiles` partial records, in FP64 and in an order
+// that depends on the sizes alone. A CTA takes 32 consecutive values of the
+// records (lane = value) and the blockIdx.y-th of gridDim.y slices of the
+// records, its kRedRows warps every kRedRows-th record of the slice; the last
+// CTA of a column of the grid to arrive adds the slices' sums in order.
+// One thread per value walking all records left a record of 97 values (one
+// per graph node) to one CTA: 16,384 of them took 0.7 to 1.1 ms, most of a
+// training step.
+constexpr int kRedRows = 8;
+constexpr int kRedCtas = 1184;  // CTAs of a reduction aimed at (eight per SM); its columns stay below this
+
+__global__ void __launch_bounds__(32 * kRedRows)
+    reduce_parts(const float* __restrict__ part, int rec, int ntiles, int slice, double* __restrict__ sums,
+                 uint32_t* __restrict__ tickets, float* __restrict__ grad, int off_w, int off_b, int nw) {
+    __shared__ double red[kRedRows][33];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
+    const int k0 = blockIdx.y * slice, k1 = min(ntiles, k0 + slice);
     double s = 0.0;
-    for (int k = 0; k < ntiles; ++k) s += part[static_cast<size_t>(k) * rec + i];
+    if (i < rec) {
+#pragma unroll 8
+        for (int k = k0 + warp; k < k1; k += kRedRows) s += part[static_cast<size_t>(k) * rec + i];
+    }
+    red[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int r = 1; r < kRedRows; ++r) s += red[r][lane];
+        if (gridDim.y > 1) {
+            sums[(static_cast<size_t>(blockIdx.x) * gridDim.y + blockIdx.y) * 32 + lane] = s;
+            __threadfence();
+            __syncwarp();
+            if (lane == 0) last = dev::ticket_arrive(tickets + blockIdx.x) == gridDim.y - 1;
+        } else if (lane == 0) {
+            last = true;
+        }
+    }
+    __syncthreads();
+    if (!last) return;
+    if (gridDim.y > 1) {
+        double t = 0.0;
+        for (int y = warp; y < static_cast<int>(gridDim.y); y += kRedRows)
+            t += __ldcg(sums + (static_cast<size_t>(blockIdx.x) * gridDim.y + y) * 32 + lane);
+        red[warp][lane] = t;
+        __syncthreads();
+        if (warp == 0) {
+            s = 0.0;
+#pragma unroll
+            for (int r = 0; r < kRedRows; ++r) s += red[r][lane];
+            if (lane == 0) tickets[blockIdx.x] = 0u;
+        }
+    }
+    if (warp != 0 || i >= rec) return;
     if (i < nw)
         grad[off_w + i] += static_cast<float>(s);
     else if (off_b >= 0)
@@ -920,6 +967,8 @@ struct Graph {
     float *dH = nullptr, *dHn = nullptr, *dS = nullptr, *dHu = nullptr, *dHp = nullptr, *dHq = nullptr;
     float* part = nullptr;
     size_t part_floats = 0;
+    double* part_sums = nullptr;      // reduce_parts: slice sums and arrival counters
+    uint32_t* part_tickets = nullptr;
     float *pw = nullptr, *pu = nullptr, *pv = nullptr, *pdv = nullptr, *pdu = nullptr;
     double* red = nullptr;  // [0..3] results, [8..] partials
     uint32_t* ticket = nullptr;
@@ -1114,7 +1163,7 @@ bool ensure_graph_buffers(Graph& gr, uint32_t n, uint32_t nnz) {
 
 // The training layout of the current graph: every layer's activations kept
 // for the backward pass, the pre-activations Au and the gradient buffers.
-bool ensure_training_buffers(Graph& gr) {
+bool ensure_training_buffers(Graph& gr, cudaStream_t s) {
     if (gr.train_arena != nullptr) return true;
     const size_t n = gr.cap_n, nl = gr.cap_nnz, nh = n * H, nho = n * HO;
     const size_t tiles = nblk(n, kRows);
@@ -1135,6 +1184,8 @@ bool ensure_training_buffers(Graph& gr) {
         c.take(t.dHp, nho);
         c.take(t.dHq, nho);
         c.take(t.part, part_floats);
+        c.take(t.part_sums, size_t(kRedCtas) * 32);
+        c.take(t.part_tickets, kRedCtas);
         c.take(t.pw, n);
         c.take(t.pu, n);
         c.take(t.pv, n);
@@ -1142,6 +1193,11 @@ bool ensure_training_buffers(Graph& gr) {
         c.take(t.pdu, n);
     });
     if (!ok) return false;
+    if (cudaMemsetAsync(t.part_tickets, 0, kRedCtas * sizeof(uint32_t), s) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(t.train_arena);
+        return false;
+    }
     t.part_floats = part_floats;
     gr = t;
     return true;
@@ -1348,7 +1404,13 @@ double loss_and_dg(_clsparseB200Spai* net, const float* probes, int K, double la
 }
 
 void reduce_into(_clsparseB200Spai* net, int rec, int ntiles, int off_w, int off_b, int nw, cudaStream_t s) {
-    reduce_parts<<<nblk(rec, 256), 256, 0, s>>>(net->gr.part, rec, ntiles, net->grad, off_w, off_b, nw);
+    // as many slices as fill the device, of 32 records or more: groups * slices <= kRedCtas
+    static_assert((H * 2 * H + H + 31) / 32 <= kRedCtas, "a record has at most 32 * kRedCtas values");
+    const uint32_t groups = nblk(rec, 32);
+    const uint32_t slices = std::max(1u, std::min<uint32_t>(kRedCtas / groups, nblk(ntiles, 32)));
+    const int slice = static_cast<int>(nblk(ntiles, static_cast<int>(slices)));
+    reduce_parts<<<dim3(groups, nblk(ntiles, slice)), 32 * kRedRows, 0, s>>>(
+        net->gr.part, rec, ntiles, slice, net->gr.part_sums, net->gr.part_tickets, net->grad, off_w, off_b, nw);
 }
 
 void backward(_clsparseB200Spai* net, int bf16, cudaStream_t s) {
@@ -1528,7 +1590,7 @@ clsparseStatus clsparseB200SpaiLossGrad(clsparseB200Spai net, const cldenseVecto
     if (st != clsparseSuccess) return st;
     if (K > 0 && (!probes || probes->num_values < size_t(K) * net->gr.n)) return clsparseInvalidSize;
     DeviceGuard g(control->device);
-    if (!ensure_training_buffers(net->gr)) return clsparseOutOfResources;
+    if (!ensure_training_buffers(net->gr, control->stream)) return clsparseOutOfResources;
     st = ensure_blocks(net->gr, control->stream);
     if (st != clsparseSuccess) return st;
     const int bf16 = fp32Weights ? 0 : 1;

@@ -38,6 +38,25 @@ def test_gpu_loss_and_gradient_match_oracle(ctrl):
     spai.release()
 
 
+@pytest.mark.parametrize("m", [2, 3, 17, 33, 57])
+def test_gradient_sizes(ctrl, m):
+    """The gradient's record sums at every split: below one slice (4 and 9
+    graph nodes), one slice, several, and a last one that is not full. The
+    same bar as above: FP32 forward and backward against FP64."""
+    (rp, c, v), A, spai = _setup(ctrl, m=m, seed=m)
+    gr = go.Graph(rp, c, v)
+    probes = np.random.default_rng(m).normal(size=(1, gr.n))
+    Lo, go_grad = go.loss_grad(spai.params().astype(np.float64), gr, list(probes), 0.3)
+    t = torch.tensor(probes, dtype=torch.float32, device="cuda")
+    Lg, gg = spai.loss_grad(ctrl, t, 0.3, fp32_weights=True)
+    assert abs(Lg - Lo) <= 1e-4 * max(1.0, abs(Lo)), (Lg, Lo)
+    rel = np.linalg.norm(gg - go_grad) / np.linalg.norm(go_grad)
+    assert rel <= 2e-3, rel
+    _, again = spai.loss_grad(ctrl, t, 0.3, fp32_weights=True)
+    np.testing.assert_array_equal(gg, again)
+    spai.release()
+
+
 def test_bf16_weights_close_to_fp32(ctrl):
     (rp, c, v), A, spai = _setup(ctrl, m=16, seed=5)
     L32, g32 = spai.loss_grad(ctrl, fp32_weights=True)
