@@ -3,29 +3,29 @@
 // counterpart.
 //
 // The systems are stacked block-diagonally in one CSR matrix (rows and columns
-// of system s are [off[s], off[s+1])). A persistent kernel keeps one CTA per
-// resident slot; each CTA takes the next system from a device work queue
-// (atomic counter over the systems ordered by decreasing nonzeros, so the
-// largest start first) and runs CG on it to completion: FP32 vectors and FP32
-// matrix values, CTA-wide reductions, no grid synchronisation and no host
-// round trip. When the recursive FP32 residual meets the tolerance, the CTA
-// recomputes the true residual b - A x in FP64; if that check fails, CG
-// restarts from the current x with the FP64 residual (refinement) until the
-// check passes or the iteration budget is spent. When every system is banded
-// (at most kBatchDiags column offsets, all inside its own rows), the products
-// come from a per-system diagonal-storage copy laid out at every call: one
-// thread per row, the values and the vector entries independent loads
-// instead of the row-pointer / column-index / vector chain of CSR, and rows
-// whose whole stencil lies inside the system without clamps (C4, 4096 stencil
-// systems: 0.349 -> 0.312 -> 0.229 s; the update pass issuing each row's
-// loads before its stores: 0.198 s; the vector passes two rows at a time:
-// 0.169 s; the product pass too: 0.165 s). Otherwise each system's SpMV uses the
-// lanes-per-row width the tuning table gives for its size class. The kernel
-// is held to two CTAs per SM (64 registers): the diagonal loop would
-// otherwise take 128 registers and halve the resident CTAs (0.51 s).
+// of system s are [off[s], off[s+1])). Each runs CG to completion on its own:
+// FP32 vectors and FP32 matrix values, no grid synchronisation and no host
+// round trip. When the recursive FP32 residual meets the tolerance, the true
+// residual b - A x is recomputed in FP64; if that check fails, CG restarts
+// from the current x with the FP64 residual (refinement) until the check
+// passes or the iteration budget is spent.
 //
-// The whole solve (queue reset, kernel) is captured once into a CUDA graph per
-// control and relaunched for repeated solves on the same operands.
+// Banded systems (at most kBatchDiags column offsets, all inside their own
+// rows; the offsets are found on the device at every call) that fit on chip
+// are solved by the resident kernel (batched_resident.cuh), one launch per
+// cluster size on streams of their own, the largest systems first.
+//
+// The others run in the persistent general kernel: one CTA per resident slot
+// takes the next system from a device work queue (largest first). When all of
+// them are banded (systems too large for a cluster's shared memory), their
+// products come from a per-system diagonal-storage copy laid out at every
+// call: one thread per row, the values and the vector entries independent
+// loads instead of the row-pointer / column-index / vector chain of CSR, and
+// rows whose whole stencil lies inside the system without clamps; otherwise
+// each system's SpMV uses the lanes-per-row width the tuning table gives for
+// its size class. The kernel is held to two CTAs per SM (64 registers): the
+// diagonal loop would otherwise take 128 registers and halve the resident
+// CTAs.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -41,10 +41,17 @@ namespace clsp {
 namespace {
 
 constexpr int kThreads = 512;
-constexpr int kWarps = kThreads / 32;
 
 // Diagonals a system may have to be solved from diagonal storage.
 constexpr int kBatchDiags = 8;
+
+}  // namespace
+}  // namespace clsp
+
+#include "batched_resident.cuh"
+
+namespace clsp {
+namespace {
 
 struct BatchArgs {
     const float* vals;
@@ -301,69 +308,104 @@ __global__ void __launch_bounds__(kThreads, 2) batched_cg_kernel(BatchArgs a) {
     }
 }
 
-// One CTA per system: the distinct column offsets col - row of its rows,
-// increasing, into doffs[s * kBatchDiags ...] and their count into dnd[s]
-// (0 when the system does not qualify); bad[0] = 1 when a system has more
-// than kBatchDiags of them, a column outside its own rows, or columns not
-// strictly increasing in a row.
-__global__ void batch_dia_detect_kernel(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ cols,
-                                        const uint32_t* __restrict__ off, int32_t* doffs, uint8_t* dnd, int* bad) {
-    constexpr int32_t kEmptySlot = INT32_MIN;  // below any offset of a system of fewer than 2^31 rows
-    __shared__ int32_t set[kBatchDiags];
-    __shared__ int over;
-    const uint32_t s = blockIdx.x;
-    const uint32_t r0 = off[s], r1 = off[s + 1];
-    if (threadIdx.x < kBatchDiags) set[threadIdx.x] = kEmptySlot;
-    if (threadIdx.x == 0) over = 0;
-    __syncthreads();
-    int mine = 0;
-    for (uint32_t row = r0 + threadIdx.x; row < r1; row += blockDim.x) {
-        for (uint32_t k = rp[row]; k < rp[row + 1]; ++k) {
-            const uint32_t c = cols[k];
-            if (c < r0 || c >= r1 || (k > rp[row] && c <= cols[k - 1])) {
-                mine = 1;
-                continue;
-            }
-            const int32_t o = static_cast<int32_t>(static_cast<int64_t>(c) - static_cast<int64_t>(row));
-            bool placed = false;
-            for (int t = 0; t < kBatchDiags && !placed; ++t) {
-                const int32_t cur = *reinterpret_cast<volatile int32_t*>(&set[t]);
-                if (cur == o) {
-                    placed = true;
-                } else if (cur == kEmptySlot) {
-                    const int32_t old = atomicCAS(&set[t], kEmptySlot, o);
-                    placed = old == kEmptySlot || old == o;
-                }
-            }
-            if (!placed) mine = 1;
+// The distinct column offsets col - row of system blockIdx.x's rows
+// [blockIdx.y * kDetectRows, ...) into its set (kBatchDiags slots preset to
+// kNoOffset); over[s] = 1 when there are more, a column lies outside the
+// system's rows, or columns are not strictly increasing in a row. A thread
+// keeps the offsets it knows to be in the set in registers and goes to the
+// shared set only for a new one (one CTA per system with every entry probing
+// the set took 2.3 ms for 1024 systems of up to 50,000 rows).
+constexpr int32_t kNoOffset = INT32_MIN;  // below any offset of a system of fewer than 2^31 rows
+constexpr uint32_t kDetectRows = 4096;
+
+__device__ __forceinline__ bool offset_insert(int32_t* set, int32_t o) {
+    for (int t = 0; t < kBatchDiags; ++t) {
+        const int32_t cur = *reinterpret_cast<volatile int32_t*>(&set[t]);
+        if (cur == o) return true;
+        if (cur == kNoOffset) {
+            const int32_t old = atomicCAS(&set[t], kNoOffset, o);
+            if (old == kNoOffset || old == o) return true;
         }
     }
-    if (mine) atomicExch(&over, 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int32_t v[kBatchDiags];
-        int nd = 0;
-        for (int t = 0; t < kBatchDiags; ++t)
-            if (set[t] != kEmptySlot) v[nd++] = set[t];
-        if (over) nd = 0;
-        for (int t = 1; t < nd; ++t)  // insertion sort of at most kBatchDiags values
-            for (int u = t; u > 0 && v[u - 1] > v[u]; --u) {
-                const int32_t w = v[u];
-                v[u] = v[u - 1];
-                v[u - 1] = w;
-            }
-        for (int t = 0; t < kBatchDiags; ++t) doffs[s * kBatchDiags + t] = t < nd ? v[t] : 0;
-        dnd[s] = static_cast<uint8_t>(nd);
-        if (over) atomicExch(bad, 1);
-    }
+    return false;
 }
 
-// One CTA per system: its CSR values into diagonal storage (dv zeroed before).
+__global__ void __launch_bounds__(256)
+    batch_dia_detect_kernel(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ cols,
+                            const uint32_t* __restrict__ off, int32_t* sets, int* over) {
+    __shared__ int32_t set[kBatchDiags];
+    const uint32_t s = blockIdx.x;
+    const uint32_t r0 = off[s], r1 = off[s + 1];
+    const uint64_t begin = r0 + static_cast<uint64_t>(blockIdx.y) * kDetectRows;
+    if (begin >= r1) return;
+    const uint32_t end = static_cast<uint32_t>(min(static_cast<uint64_t>(r1), begin + kDetectRows));
+    if (threadIdx.x < kBatchDiags) set[threadIdx.x] = kNoOffset;
+    __syncthreads();
+    bool bad = false;
+    int32_t known[kBatchDiags];
+#pragma unroll
+    for (int t = 0; t < kBatchDiags; ++t) known[t] = kNoOffset;
+    for (uint32_t row = static_cast<uint32_t>(begin) + threadIdx.x; row < end; row += blockDim.x) {
+        const uint32_t kb = rp[row], ke = rp[row + 1];
+        uint32_t prev = 0;
+        for (uint32_t k = kb; k < ke; ++k) {
+            const uint32_t c = cols[k];
+            if (c < r0 || c >= r1 || (k > kb && c <= prev)) {
+                bad = true;
+            } else {
+                const int32_t o = static_cast<int32_t>(static_cast<int64_t>(c) - static_cast<int64_t>(row));
+                bool seen = false;
+#pragma unroll
+                for (int t = 0; t < kBatchDiags; ++t) seen |= known[t] == o;
+                if (!seen) {
+                    bad |= !offset_insert(set, o);
+#pragma unroll
+                    for (int t = 0; t < kBatchDiags; ++t) known[t] = *reinterpret_cast<volatile int32_t*>(&set[t]);
+                }
+            }
+            prev = c;
+        }
+    }
+    if (bad) atomicOr(over + s, 1);
+    __syncthreads();
+    if (threadIdx.x < kBatchDiags && set[threadIdx.x] != kNoOffset &&
+        !offset_insert(sets + static_cast<size_t>(s) * kBatchDiags, set[threadIdx.x]))
+        atomicOr(over + s, 1);
+}
+
+// The sets sorted: offsets of system s increasing at doffs[s * kBatchDiags],
+// their number in dnd[s] (0: not banded, or no entries).
+__global__ void batch_dia_sort_kernel(int32_t* doffs, const int* over, uint8_t* dnd, uint32_t nsys) {
+    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= nsys) return;
+    int32_t v[kBatchDiags];
+    int nd = 0;
+    int32_t* o = doffs + static_cast<size_t>(s) * kBatchDiags;
+    for (int t = 0; t < kBatchDiags; ++t)
+        if (o[t] != kNoOffset) v[nd++] = o[t];
+    if (over[s]) nd = 0;
+    for (int t = 1; t < nd; ++t)  // insertion sort of at most kBatchDiags values
+        for (int u = t; u > 0 && v[u - 1] > v[u]; --u) {
+            const int32_t w = v[u];
+            v[u] = v[u - 1];
+            v[u - 1] = w;
+        }
+    for (int t = 0; t < kBatchDiags; ++t) o[t] = t < nd ? v[t] : 0;
+    dnd[s] = static_cast<uint8_t>(nd);
+}
+
+__global__ void fill_i32_kernel(int32_t* p, size_t n, int32_t v) {
+    const size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i < n) p[i] = v;
+}
+
+// One CTA per system of `list`: its CSR values into diagonal storage (dv
+// zeroed before).
 __global__ void batch_dia_fill_kernel(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ cols,
                                       const float* __restrict__ vals, const uint32_t* __restrict__ off,
-                                      const int32_t* __restrict__ doffs, const uint8_t* __restrict__ dnd,
+                                      const uint32_t* __restrict__ list, const int32_t* __restrict__ doffs, const uint8_t* __restrict__ dnd,
                                       const uint64_t* __restrict__ dbase, float* dv) {
-    const uint32_t s = blockIdx.x;
+    const uint32_t s = list[blockIdx.x];
     const uint32_t r0 = off[s], r1 = off[s + 1], ns = r1 - r0;
     const int nd = dnd[s];
     const int32_t* o = doffs + s * kBatchDiags;
@@ -388,6 +430,71 @@ int default_lanes(uint32_t n, uint32_t nnz) {
     if (per >= 24) return 8;
     if (per >= 12) return 4;
     return 2;
+}
+
+// ---- which systems the resident kernel takes, and how
+
+constexpr int kResWide = 512;   // threads of a CTA, one CTA per SM
+constexpr int kResSmall = 128;  // systems of up to 128 * kResRows rows: several CTAs per SM
+
+// Shared memory a resident CTA may ask for: the 227 KB of an SM less the
+// kernel's static part (the exchange's slots) and the CTA's reserve.
+constexpr size_t kResSmem = 218 * 1024;
+
+// One launch of the resident kernel: systems solved by clusters of the same size.
+struct ResidentClass {
+    int threads = 0, cluster = 0;
+    size_t smem = 0;               // the largest of its systems
+    std::vector<uint32_t> list;    // largest first
+};
+
+// Whether a system of n rows with nd sorted offsets runs on C CTAs of NT
+// threads: its rows in the registers, its diagonals in shared memory, and its
+// stencil reaching no further than the neighbouring CTA.
+bool resident_fits(uint32_t n, const int32_t* off, int nd, uint32_t C, uint32_t NT, size_t& smem) {
+    const uint64_t m = (static_cast<uint64_t>(n) + C - 1) / C;
+    const uint64_t lo = off[0] < 0 ? static_cast<uint64_t>(-static_cast<int64_t>(off[0])) : 0;
+    const uint64_t hi = off[nd - 1] > 0 ? static_cast<uint64_t>(off[nd - 1]) : 0;
+    if (m > static_cast<uint64_t>(NT) * kResRows || (C > 1 && (lo > m || hi > m))) return false;
+    smem = resident_smem(m, nd, lo, hi);
+    return smem <= kResSmem;
+}
+
+template <int NT>
+cudaError_t launch_resident(const ResidentArgs& a, const ResidentClass& k, cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(batched_resident_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(kResSmem));
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<uint32_t>(k.list.size()) * static_cast<uint32_t>(k.cluster));
+    cfg.blockDim = dim3(NT);
+    cfg.dynamicSmemBytes = k.smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<uint32_t>(k.cluster);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, batched_resident_kernel<NT>, a);
+}
+
+// Streams and events of the resident launches, made on first use.
+bool ensure_streams(BatchWork& w, size_t count) {
+    if (!w.begin && cudaEventCreateWithFlags(&w.begin, cudaEventDisableTiming) != cudaSuccess) return false;
+    while (w.streams.size() < count) {
+        cudaStream_t s = nullptr;
+        cudaEvent_t e = nullptr;
+        if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return false;
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+            cudaStreamDestroy(s);
+            return false;
+        }
+        w.streams.push_back(s);
+        w.ends.push_back(e);
+    }
+    return true;
 }
 
 }  // namespace
@@ -422,7 +529,7 @@ clsparseStatus clsparseScsrcgBatched(cldenseVector* x, const clsparseCsrMatrix* 
     const size_t vb = ((n * 4 + 255) / 256) * 256;
     const size_t meta_bytes = 16 + (nsys + 1) * 4 * 2 + nsys * 4 + nsys + 256;
     const size_t out_bytes = nsys * (4 + 8 + 4) + 64;
-    if (w.vecs.ensure(4 * vb + 256) != cudaSuccess || w.meta.ensure(meta_bytes) != cudaSuccess ||
+    if (w.meta.ensure(meta_bytes) != cudaSuccess ||
         w.out.ensure(out_bytes) != cudaSuccess) {
         cudaGetLastError();
         return clsparseOutOfResources;
@@ -454,128 +561,197 @@ clsparseStatus clsparseScsrcgBatched(cldenseVector* x, const clsparseCsrMatrix* 
         if (l != 1 && l != 2 && l != 4 && l != 8 && l != 16 && l != 32) return clsparseInvalidValue;
         lanes[k] = static_cast<uint8_t>(l);
     }
-    cudaMemcpyAsync(d_order, order.data(), nsys * 4, cudaMemcpyHostToDevice, s);
     cudaMemcpyAsync(d_lanes, lanes.data(), nsys, cudaMemcpyHostToDevice, s);
 
-    // Diagonal storage when every system is banded (at most kBatchDiags
-    // column offsets inside its own rows): offsets found on the device, the
-    // values laid out by diagonal at every call (so values changed in place
-    // are seen). CLSPARSE_B200_BATCH_DIA=0 keeps every system on CSR.
-    const float* dvals = nullptr;
-    const uint64_t* d_dbase = nullptr;
-    const int32_t* d_doffs = nullptr;
-    const uint8_t* d_dnd = nullptr;
+    // Offsets of every system, found on the device at every call (so a matrix
+    // changed in place is seen). CLSPARSE_B200_BATCH_DIA=0 keeps every system
+    // on CSR.
     const char* dia_env = std::getenv("CLSPARSE_B200_BATCH_DIA");
-    if (!(dia_env && std::atoi(dia_env) == 0)) {
-        const size_t offs_b = ((static_cast<size_t>(nsys) * kBatchDiags * 4 + 255) / 256) * 256;
+    const bool dia = !(dia_env && std::atoi(dia_env) == 0);
+    std::vector<uint8_t> hnd(nsys, 0);
+    std::vector<int32_t> hoffs;
+    int32_t* doffs = nullptr;
+    uint64_t* dbase = nullptr;
+    uint8_t* dnd = nullptr;
+    const uint32_t* cols = dev_ptr<const uint32_t>(A->col_indices, A->off_col_indices);
+    if (dia) {
+        const size_t noff = static_cast<size_t>(nsys) * kBatchDiags;
+        const size_t offs_b = ((noff * 4 + 255) / 256) * 256;
         const size_t base_b = ((static_cast<size_t>(nsys) * 8 + 255) / 256) * 256;
-        const size_t nd_b = ((static_cast<size_t>(nsys) + 255) / 256) * 256;
-        if (w.dia_meta.ensure(offs_b + base_b + nd_b + 256) != cudaSuccess) {
+        const size_t over_b = ((static_cast<size_t>(nsys) * 4 + 255) / 256) * 256;
+        if (w.dia_meta.ensure(offs_b + base_b + over_b + nsys + 256) != cudaSuccess) {
             cudaGetLastError();
             return clsparseOutOfResources;
         }
         char* dm = static_cast<char*>(w.dia_meta.ptr);
-        int32_t* doffs = reinterpret_cast<int32_t*>(dm);
-        uint64_t* dbase = reinterpret_cast<uint64_t*>(dm + offs_b);
-        uint8_t* dnd = reinterpret_cast<uint8_t*>(dm + offs_b + base_b);
-        int* bad = reinterpret_cast<int*>(dm + offs_b + base_b + nd_b);
-        const uint32_t* cols = dev_ptr<const uint32_t>(A->col_indices, A->off_col_indices);
-        cudaMemsetAsync(bad, 0, sizeof(int), s);
-        batch_dia_detect_kernel<<<nsys, 256, 0, s>>>(rp, cols, d_off, doffs, dnd, bad);
-        std::vector<uint8_t> hnd(nsys);
-        int hbad = 1;
-        cudaMemcpyAsync(hnd.data(), dnd, nsys, cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, s);
-        if (cudaStreamSynchronize(s) != cudaSuccess) return clsparseInvalidKernelExecution;
-        if (hbad == 0) {
-            std::vector<uint64_t> hbase(nsys);
+        doffs = reinterpret_cast<int32_t*>(dm);
+        dbase = reinterpret_cast<uint64_t*>(dm + offs_b);
+        int* over = reinterpret_cast<int*>(dm + offs_b + base_b);
+        dnd = reinterpret_cast<uint8_t*>(dm + offs_b + base_b + over_b);
+        uint32_t largest = 1;
+        for (uint32_t k = 0; k < nsys; ++k) largest = std::max(largest, off[k + 1] - off[k]);
+        const uint32_t chunks = std::min<uint32_t>((largest - 1) / kDetectRows + 1, 65535u);
+        fill_i32_kernel<<<static_cast<uint32_t>((noff + 255) / 256), 256, 0, s>>>(doffs, noff, kNoOffset);
+        cudaMemsetAsync(over, 0, static_cast<size_t>(nsys) * 4, s);
+        if (static_cast<uint64_t>(chunks) * kDetectRows >= largest) {
+            batch_dia_detect_kernel<<<dim3(nsys, chunks), 256, 0, s>>>(rp, cols, d_off, doffs, over);
+            batch_dia_sort_kernel<<<(nsys + 255) / 256, 256, 0, s>>>(doffs, over, dnd, nsys);
+            hoffs.resize(noff);
+            cudaMemcpyAsync(hnd.data(), dnd, nsys, cudaMemcpyDeviceToHost, s);
+            cudaMemcpyAsync(hoffs.data(), doffs, noff * 4, cudaMemcpyDeviceToHost, s);
+            if (cudaStreamSynchronize(s) != cudaSuccess) return clsparseInvalidKernelExecution;
+        }
+    }
+
+    // Systems of the resident kernel by CTA width and cluster size: the
+    // smallest cluster that holds the system takes the least SM time (the
+    // exchanges cost every CTA of a cluster alike); while the batch leaves
+    // SMs idle, all clusters are doubled.
+    std::vector<ResidentClass> classes(5);
+    const int sizes[5][2] = {{kResWide, 8}, {kResWide, 4}, {kResWide, 2}, {kResWide, 1}, {kResSmall, 1}};
+    for (int k = 0; k < 5; ++k) {
+        classes[k].threads = sizes[k][0];
+        classes[k].cluster = sizes[k][1];
+    }
+    std::vector<int> at(nsys, -1);  // class of each system, -1: the general kernel
+    auto place = [&](uint32_t k, int c) {
+        size_t need = 0;
+        return hnd[k] > 0 && resident_fits(off[k + 1] - off[k], &hoffs[static_cast<size_t>(k) * kBatchDiags], hnd[k],
+                                           static_cast<uint32_t>(sizes[c][1]), static_cast<uint32_t>(sizes[c][0]), need)
+                   ? need
+                   : size_t(0);
+    };
+    uint64_t ctas = 0;
+    for (uint32_t k = 0; k < nsys; ++k)
+        for (int c = 4; c >= 0 && at[k] < 0; --c)
+            if (place(k, c)) {
+                at[k] = c;
+                ctas += static_cast<uint64_t>(sizes[c][1]);
+            }
+    for (int step = 0; step < 4 && ctas > 0 && 2 * ctas <= static_cast<uint64_t>(control->sm_count); ++step) {
+        ctas = 0;
+        for (uint32_t k = 0; k < nsys; ++k) {
+            if (at[k] > 0 && place(k, at[k] - 1)) --at[k];
+            if (at[k] >= 0) ctas += static_cast<uint64_t>(sizes[at[k]][1]);
+        }
+    }
+    std::vector<uint32_t> lists, rest;  // device lists: the classes one after another, then the rest
+    for (uint32_t k : order) {
+        if (at[k] < 0) {
+            rest.push_back(k);
+            continue;
+        }
+        classes[at[k]].list.push_back(k);
+        classes[at[k]].smem = std::max(classes[at[k]].smem, place(k, at[k]));
+    }
+    for (const ResidentClass& c : classes) lists.insert(lists.end(), c.list.begin(), c.list.end());
+    const size_t rest_at = lists.size();
+    lists.insert(lists.end(), rest.begin(), rest.end());
+    cudaMemcpyAsync(d_order, lists.data(), nsys * 4, cudaMemcpyHostToDevice, s);
+
+    char* ob = static_cast<char*>(w.out.ptr);
+    double* d_residual = reinterpret_cast<double*>(ob);
+    int* d_iters = reinterpret_cast<int*>(ob + nsys * 8);
+    int* d_converged = reinterpret_cast<int*>(ob + nsys * 12);
+    const float* vals = dev_ptr<const float>(A->values, A->off_values);
+    float* xp = dev_ptr<float>(x->values, x->off_values);
+    const float* bp = dev_ptr<const float>(b->values, b->off_values);
+
+    bool failed = false;
+    size_t forked = 0;
+    if (rest_at > 0) {
+        // each class on a stream of its own, after what the caller's stream holds
+        size_t used = 0;
+        for (const ResidentClass& c : classes) used += c.list.empty() ? 0 : 1;
+        if (!ensure_streams(w, used) || cudaEventRecord(w.begin, s) != cudaSuccess) {
+            cudaGetLastError();
+            return clsparseOutOfResources;
+        }
+        ResidentArgs ra{vals, cols, rp,    xp,      bp,         d_off,       d_order,
+                        doffs, dnd, d_iters, d_residual, d_converged, solverControl->maxIters,
+                        solverControl->relativeTolerance};
+        for (const ResidentClass& c : classes) {
+            if (c.list.empty()) continue;
+            cudaStream_t cs = w.streams[forked];
+            failed |= cudaStreamWaitEvent(cs, w.begin, 0) != cudaSuccess;
+            failed |= (c.threads == kResWide ? launch_resident<kResWide>(ra, c, cs)
+                                             : launch_resident<kResSmall>(ra, c, cs)) != cudaSuccess;
+            failed |= cudaEventRecord(w.ends[forked], cs) != cudaSuccess;
+            ++forked;
+            ra.list += c.list.size();
+            if (failed) break;
+        }
+    }
+    if (!rest.empty() && !failed) {
+        const uint32_t nrest = static_cast<uint32_t>(rest.size());
+        bool banded = dia;
+        for (uint32_t k : rest) banded = banded && hnd[k] > 0;
+        if (w.vecs.ensure(4 * vb + 256) != cudaSuccess) failed = true;
+        BatchArgs a;
+        std::memset(&a, 0, sizeof(a));
+        if (banded && !failed) {
+            std::vector<uint64_t> hbase(nsys, 0);
             uint64_t total = 0;
-            for (uint32_t k = 0; k < nsys; ++k) {
+            for (uint32_t k : rest) {
                 hbase[k] = total;
                 total += static_cast<uint64_t>(hnd[k]) * (off[k + 1] - off[k]);
             }
             if (w.dia.ensure(total * sizeof(float) + 256) != cudaSuccess) {
-                cudaGetLastError();
-                return clsparseOutOfResources;
+                failed = true;
+            } else {
+                cudaMemcpyAsync(dbase, hbase.data(), nsys * 8, cudaMemcpyHostToDevice, s);
+                cudaMemsetAsync(w.dia.ptr, 0, total * sizeof(float), s);
+                batch_dia_fill_kernel<<<nrest, 256, 0, s>>>(rp, cols, vals, d_off, d_order + rest_at, doffs, dnd, dbase,
+                                                            static_cast<float*>(w.dia.ptr));
+                a.dvals = static_cast<const float*>(w.dia.ptr);
+                a.dbase = dbase;
+                a.doffs = doffs;
+                a.dnd = dnd;
             }
-            cudaMemcpyAsync(dbase, hbase.data(), nsys * 8, cudaMemcpyHostToDevice, s);
-            cudaMemsetAsync(w.dia.ptr, 0, total * sizeof(float), s);
-            batch_dia_fill_kernel<<<nsys, 256, 0, s>>>(rp, cols, dev_ptr<const float>(A->values, A->off_values), d_off,
-                                                      doffs, dnd, dbase, static_cast<float*>(w.dia.ptr));
-            if (cudaGetLastError() != cudaSuccess) return clsparseInvalidKernelExecution;
-            dvals = static_cast<const float*>(w.dia.ptr);
-            d_dbase = dbase;
-            d_doffs = doffs;
-            d_dnd = dnd;
+        }
+        if (!failed) {
+            a.vals = vals;
+            a.cols = cols;
+            a.rp = rp;
+            a.x = xp;
+            a.b = bp;
+            char* vbase = static_cast<char*>(w.vecs.ptr);
+            a.r = reinterpret_cast<float*>(vbase);
+            a.p = reinterpret_cast<float*>(vbase + vb);
+            a.q = reinterpret_cast<float*>(vbase + 2 * vb);
+            a.invd = reinterpret_cast<float*>(vbase + 3 * vb);
+            a.off = d_off;
+            a.order = d_order + rest_at;
+            a.lanes = d_lanes;
+            a.counter = d_counter;
+            a.residual = d_residual;
+            a.iters = d_iters;
+            a.converged = d_converged;
+            a.nsys = nrest;
+            a.max_iters = solverControl->maxIters;
+            a.tol = solverControl->relativeTolerance;
+            int per_sm = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batched_cg_kernel, kThreads, 0);
+            const uint32_t grid = std::min(static_cast<uint32_t>(control->sm_count * std::max(per_sm, 1)), nrest);
+            cudaMemsetAsync(d_counter, 0, 16, s);
+            batched_cg_kernel<<<grid, kThreads, 0, s>>>(a);
+            failed |= cudaGetLastError() != cudaSuccess;
         }
     }
-
-    char* ob = static_cast<char*>(w.out.ptr);
-    static_assert(sizeof(BatchArgs) <= sizeof(w.args), "argument record");
-    BatchArgs a;
-    std::memset(&a, 0, sizeof(a));
-    a.vals = dev_ptr<const float>(A->values, A->off_values);
-    a.cols = dev_ptr<const uint32_t>(A->col_indices, A->off_col_indices);
-    a.rp = rp;
-    a.x = dev_ptr<float>(x->values, x->off_values);
-    a.b = dev_ptr<const float>(b->values, b->off_values);
-    char* vbase = static_cast<char*>(w.vecs.ptr);
-    a.r = reinterpret_cast<float*>(vbase);
-    a.p = reinterpret_cast<float*>(vbase + vb);
-    a.q = reinterpret_cast<float*>(vbase + 2 * vb);
-    a.invd = reinterpret_cast<float*>(vbase + 3 * vb);
-    a.off = d_off;
-    a.order = d_order;
-    a.lanes = d_lanes;
-    a.counter = d_counter;
-    a.residual = reinterpret_cast<double*>(ob);
-    a.iters = reinterpret_cast<int*>(ob + nsys * 8);
-    a.converged = reinterpret_cast<int*>(ob + nsys * 12);
-    a.nsys = nsys;
-    a.max_iters = solverControl->maxIters;
-    a.tol = solverControl->relativeTolerance;
-    a.dvals = dvals;
-    a.dbase = d_dbase;
-    a.doffs = d_doffs;
-    a.dnd = d_dnd;
-
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batched_cg_kernel, kThreads, 0);
-    uint32_t grid = static_cast<uint32_t>(control->sm_count * std::max(per_sm, 1));
-    grid = std::min(grid, nsys);
-
-    // One graph per operand set: reset the queue, run the persistent kernel.
-    const bool same = w.exec && w.grid == grid && std::memcmp(&w.args, &a, sizeof(a)) == 0;
-    if (!same) {
-        if (w.exec) cudaGraphExecDestroy(w.exec);
-        w.exec = nullptr;
-        cudaStream_t cs = control->capture_stream;
-        cudaGraph_t graph = nullptr;
-        if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
-            return clsparseInvalidKernelExecution;
-        cudaMemsetAsync(d_counter, 0, 16, cs);
-        batched_cg_kernel<<<grid, kThreads, 0, cs>>>(a);
-        if (cudaStreamEndCapture(cs, &graph) != cudaSuccess) {
-            cudaGetLastError();
-            return clsparseInvalidKernelExecution;
-        }
-        const cudaError_t ie = cudaGraphInstantiate(&w.exec, graph, 0);
-        cudaGraphDestroy(graph);
-        if (ie != cudaSuccess) {
-            w.exec = nullptr;
-            cudaGetLastError();
-            return clsparseInvalidKernelExecution;
-        }
-        std::memcpy(&w.args, &a, sizeof(a));
-        w.grid = grid;
+    for (size_t k = 0; k < forked; ++k) failed |= cudaStreamWaitEvent(s, w.ends[k], 0) != cudaSuccess;
+    if (failed) {
+        // nothing of this call stays in flight on the buffers
+        cudaGetLastError();
+        for (size_t k = 0; k < forked; ++k) cudaStreamSynchronize(w.streams[k]);
+        cudaStreamSynchronize(s);
+        return clsparseInvalidKernelExecution;
     }
-    if (cudaGraphLaunch(w.exec, s) != cudaSuccess) return clsparseInvalidKernelExecution;
 
     std::vector<double> res(nsys);
     std::vector<int> its(nsys), conv(nsys);
-    cudaMemcpyAsync(res.data(), a.residual, nsys * 8, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(its.data(), a.iters, nsys * 4, cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(conv.data(), a.converged, nsys * 4, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(res.data(), d_residual, nsys * 8, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(its.data(), d_iters, nsys * 4, cudaMemcpyDeviceToHost, s);
+    cudaMemcpyAsync(conv.data(), d_converged, nsys * 4, cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) return clsparseInvalidKernelExecution;
     if (control->event) cudaEventRecord(control->event, s);
     int nconv = 0, maxit = 0;

@@ -59,15 +59,18 @@ struct MixedWork {
     }
 };
 
-// Work area and cached graph of the batched solver (batched.cu).
+// Work area of the batched solver (batched.cu) and the streams its launches
+// of one call run on.
 struct BatchWork {
     DeviceBuffer vecs, meta, out;
     DeviceBuffer dia, dia_meta;  // diagonal-storage copies of banded systems and their offsets
-    cudaGraphExec_t exec = nullptr;
-    unsigned char args[256] = {};  // kernel arguments the graph was captured with
-    uint32_t grid = 0;
+    std::vector<cudaStream_t> streams;
+    std::vector<cudaEvent_t> ends;
+    cudaEvent_t begin = nullptr;
     ~BatchWork() {
-        if (exec) cudaGraphExecDestroy(exec);
+        for (cudaStream_t s : streams) cudaStreamDestroy(s);
+        for (cudaEvent_t e : ends) cudaEventDestroy(e);
+        if (begin) cudaEventDestroy(begin);
     }
 };
 

@@ -101,3 +101,77 @@ def test_batch_with_a_non_banded_system_runs_on_csr(ctrl):
         a, e = int(offs[s]), int(offs[s + 1])
         bs = b[a:e].astype(np.float64)
         assert np.linalg.norm(bs - M32[a:e, a:e] @ xs[a:e]) / np.linalg.norm(bs) <= 1.05e-6
+
+
+def _banded_spd(n, offsets, seed):
+    """Symmetric, strictly diagonally dominant matrix with the given upper
+    offsets, some entries missing (boundaries inside the system)."""
+    rng = np.random.default_rng(seed)
+    M = sp.csr_matrix((n, n))
+    for o in offsets:
+        if o < n:
+            v = -rng.uniform(0.1, 1.0, n - o) * (rng.uniform(size=n - o) < 0.9)
+            U = sp.diags([v], [o], shape=(n, n))
+            M = M + U + U.T
+    M = M + sp.diags([np.asarray(abs(M).sum(axis=1)).ravel() + rng.uniform(0.01, 0.2, n)], [0])
+    M = M.tocsr()
+    M.eliminate_zeros()
+    M.sort_indices()
+    return M
+
+
+# Rows at the edges of a CTA's registers (14 per thread: 1792, 7168), of the
+# cluster sizes 2, 4 and 8, past the largest, and of uneven splits; diagonals
+# 1 to 8; stencils that reach one row short of, exactly and past the
+# neighbouring CTA of the split.
+RESIDENT = [
+    [(1, [1]), (2, [1]), (33, [1, 5]), (128, [1, 16]), (129, [1, 2, 3])],
+    [(1791, [1]), (1792, [1, 40]), (1793, [1, 40]), (1800, [1, 899]), (1900, [1, 2, 1899])],
+    [(7167, [1, 80]), (7168, [1, 19, 361]), (7169, [1, 19, 361]), (14336, [1, 119]), (14337, [1, 24, 7168])],
+    [(28672, [1, 30, 900]), (28673, [1, 169]), (20000, [1, 4999]), (20000, [1, 5001]), (9000, [1, 2, 4])],
+    [(50001, [1, 37, 1369]), (57343, [1, 239]), (300, [1])],
+    [(57345, [1, 239]), (500, [1, 22]), (40000, [1, 30000])],
+]
+
+
+@pytest.mark.parametrize("case", range(len(RESIDENT)))
+def test_resident_sizes_against_csr(ctrl, case, monkeypatch):
+    """Systems held on chip against the general kernel's CSR path: every
+    residual recomputed here in FP64 meets the tolerance and is the reported
+    one, and the two solutions agree to the tolerance times the condition of
+    these matrices (row sums at least 1 % of the diagonal: below 1e3)."""
+    mats = [_banded_spd(n, o, seed=100 * case + k) for k, (n, o) in enumerate(RESIDENT[case])]
+    M = sp.block_diag(mats, format="csr")
+    M.sort_indices()
+    off = np.concatenate([[0], np.cumsum([m.shape[0] for m in mats])]).astype(np.uint32)
+    n = M.shape[0]
+    A = api.CsrMatrix.from_numpy(M.indptr.astype(np.uint32), M.indices.astype(np.uint32), M.data, dtype=torch.float32)
+    M32 = sp.csr_matrix((M.data.astype(np.float32).astype(np.float64), M.indices, M.indptr), shape=M.shape)
+    b = np.random.default_rng(case).uniform(-1, 1, n).astype(np.float32)
+    x0 = np.random.default_rng(case + 50).uniform(-1, 1, n).astype(np.float32)
+    xs = {}
+    for storage in ("resident", "csr"):
+        if storage == "csr":
+            monkeypatch.setenv("CLSPARSE_B200_BATCH_DIA", "0")
+        x = torch.tensor(x0, device="cuda")
+        sc = api.SolverControl(L.DIAGONAL, 5000, 1e-6, 0.0)
+        out = api.cg_batched(x, A, torch.tensor(b, device="cuda"), off, sc, ctrl)
+        # the iteration budget ends a solve between two exchanges alike
+        few = torch.tensor(x0, device="cuda")
+        sc3 = api.SolverControl(L.DIAGONAL, 3, 1e-6, 0.0)
+        out3 = api.cg_batched(few, A, torch.tensor(b, device="cuda"), off, sc3, ctrl)
+        sc.release()
+        sc3.release()
+        assert out["converged"] == len(mats), out
+        xs[storage] = x.cpu().numpy().astype(np.float64), few.cpu().numpy().astype(np.float64), out3["residuals"]
+        for s in range(len(mats)):
+            a, e = int(off[s]), int(off[s + 1])
+            bs = b[a:e].astype(np.float64)
+            res = np.linalg.norm(bs - M32[a:e, a:e] @ xs[storage][0][a:e]) / np.linalg.norm(bs)
+            assert res <= 1.05e-6 and abs(out["residuals"][s] - res) <= 1e-9 + 1e-3 * res, (storage, s, res)
+    for s in range(len(mats)):
+        a, e = int(off[s]), int(off[s + 1])
+        for k in (0, 1):
+            u, v = xs["resident"][k][a:e], xs["csr"][k][a:e]
+            assert np.linalg.norm(u - v) <= 1e-3 * np.linalg.norm(v), (s, k)
+        assert abs(xs["resident"][2][s] - xs["csr"][2][s]) <= 1e-3 * xs["csr"][2][s] + 1e-6
