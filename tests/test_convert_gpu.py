@@ -156,3 +156,46 @@ def test_coomv_sorted_with_duplicates(ctrl, dt, alpha, beta):
     scale = abs(alpha) * (abs(A) @ abs(x.astype(t).astype(np.float64))) + abs(beta * y0) + 1e-300
     tol = 1e-12 if dt == "f64" else 1e-5
     assert np.max(np.abs(yt.cpu().numpy() - ref) / scale) <= 10 * tol
+
+
+@pytest.mark.parametrize("off", [0, 1, 3])
+@pytest.mark.parametrize("dt", ["f64", "f32"])
+@pytest.mark.parametrize("rows,nnz", [(1, 1), (5, 0), (40, 2047), (40, 2048), (40, 2049), (9000, 4096), (100000, 3),
+                                      (30000, 20000), (3, 10000)])
+def test_coo_csr_runs(ctrl, dt, rows, nnz, off):
+    """Both directions around a CTA's run of 2048 nonzeros, with short and
+    long gaps of empty rows before, between and behind the nonzeros, and
+    arrays that do not start on 16 bytes: exact."""
+    dtype, t = DT[dt], NPT[dt]
+    rng = np.random.default_rng(rows + nnz)
+    r = np.sort(rng.choice(max(rows // 3, 1), nnz) + (rows // 3 if rows > 3 else 0)) if nnz else np.zeros(0, np.int64)
+    c = rng.integers(0, 777, nnz)
+    v = rng.uniform(-1, 1, nnz).astype(t)
+
+    def dev(a, d):
+        return torch.cat([torch.full((off,), 77, dtype=d, device="cuda"), torch.tensor(a, device="cuda").to(d),
+                          torch.full((4,), 78, dtype=d, device="cuda")])
+
+    ri, ci, vv = dev(r, torch.int32), dev(c, torch.int32), dev(v, dtype)
+    cm = coo_struct(ri, ci, vv, rows, 777)
+    cm.num_nonzeros = nnz
+    cm.off_values = cm.off_col_indices = cm.off_row_indices = off
+    rp, co, vo = (torch.full((off + k + 4,), 99, dtype=d, device="cuda") for k, d in
+                  ((rows + 1, torch.int32), (nnz, torch.int32), (nnz, dtype)))
+    out = api.CsrMatrix(rp, co, vo, 777)
+    out.s.off_values = out.s.off_col_indices = out.s.off_row_pointer = off
+    p = "D" if dt == "f64" else "S"
+    assert getattr(api.lib(), f"clsparse{p}coo2csr")(C.byref(cm), C.byref(out.s), ctrl.handle) == 0
+    want = np.searchsorted(r, np.arange(rows + 1), side="left")
+    for got, ref in ((rp, want), (co, c), (vo, v)):
+        g = got.cpu().numpy()
+        np.testing.assert_array_equal(g[off:off + len(ref)], ref)
+        assert (g[:off] == 99).all() and (g[off + len(ref):] == 99).all()
+    r2, c2, v2 = (torch.full((off + nnz + 4,), 55, dtype=d, device="cuda") for d in (torch.int32, torch.int32, dtype))
+    cm2 = coo_struct(r2, c2, v2, 0, 0)
+    cm2.off_values = cm2.off_col_indices = cm2.off_row_indices = off
+    assert getattr(api.lib(), f"clsparse{p}csr2coo")(C.byref(out.s), C.byref(cm2), ctrl.handle) == 0
+    for got, ref in ((r2, r), (c2, c), (v2, v)):
+        g = got.cpu().numpy()
+        np.testing.assert_array_equal(g[off:off + nnz], ref)
+        assert (g[:off] == 55).all() and (g[off + nnz:] == 55).all()
