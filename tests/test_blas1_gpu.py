@@ -115,3 +115,39 @@ def test_async_mode_and_event(ctrl):
     assert ev.status == 0 and ev.event
     torch.cuda.synchronize()
     assert float(s) == n
+
+
+@pytest.mark.parametrize("offs", [(0, 0, 0), (1, 1, 1), (3, 3, 3), (0, 1, 0), (2, 0, 2)], ids=str)
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
+@pytest.mark.parametrize("n", [1, 2, 5, 17, 4095, 4096, 4099, 606_208, 606_213, 3_000_001])
+def test_vector_runs(ctrl, dtype, n, offs):
+    """Elementwise results and reductions around a vector, a CTA's pass, one
+    wave of reduction CTAs and beyond, with operands that start alike or
+    differently off a 16-byte boundary: the elementwise ops differ from FP64 by
+    the roundings of one multiply and one add, the sums by the bars above."""
+    rng = np.random.default_rng(n)
+    ox, oy, orr = offs
+    px, py = t(rng.uniform(-1, 1, n + ox + 3), dtype), t(rng.uniform(0.5, 1, n + oy + 3), dtype)
+    pr = torch.full((n + orr + 3,), 9.0, dtype=dtype, device="cuda")
+    x, y, r = px[ox:ox + n], py[oy:oy + n], pr[orr:orr + n]
+    xd, yd = x.double().cpu().numpy(), y.double().cpu().numpy()
+    a, b = t([0.375], dtype), t([-0.75], dtype)
+    p = "D" if dtype == torch.float64 else "S"
+    eps = np.finfo(np.float64 if dtype == torch.float64 else np.float32).eps
+    for name, args, ref in ((f"cldense{p}axpy", (("s", a), x, y), yd + 0.375 * xd),
+                            (f"cldense{p}axpby", (("s", a), x, ("s", b), y), 0.375 * xd - 0.75 * yd),
+                            (f"cldense{p}scale", (("s", a), x), 0.375 * xd),
+                            (f"cldense{p}div", (x, y), xd / yd)):
+        api.blas1(name, r, *args, ctrl=ctrl)
+        got = pr.double().cpu().numpy()
+        assert np.all(np.abs(got[orr:orr + n] - ref) <= 2 * eps * (np.abs(xd) + np.abs(yd) + np.abs(ref))), name
+        assert (got[:orr] == 9).all() and (got[orr + n:] == 9).all(), name
+    api.blas1(f"cldense{p}mul", x, x, y, ctrl=ctrl)  # in place
+    assert np.all(np.abs(x.double().cpu().numpy() - xd * yd) <= eps * np.abs(xd))
+    xd = x.double().cpu().numpy()
+    s = torch.zeros(1, dtype=dtype, device="cuda")
+    for name, args, ref, scale in ((f"cldense{p}dot", (x, y), (xd * yd).sum(), np.abs(xd * yd).sum()),
+                                   (f"cldense{p}nrm1", (x,), np.abs(xd).sum(), np.abs(xd).sum()),
+                                   (f"cldense{p}nrm2", (y,), np.linalg.norm(yd), np.linalg.norm(yd))):
+        api.blas1(name, ("s", s), *args, ctrl=ctrl)
+        assert abs(float(s) - ref) <= TOL[dtype] * scale + 1e-300, name
