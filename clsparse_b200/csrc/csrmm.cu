@@ -17,7 +17,7 @@
 // then the loads in flight. Measured, 200,003 rows of log-normal lengths
 // (5.0 M nonzeros, uniform columns), FP32, 40 columns: 934 us with one lane
 // per column and one dependent load per nonzero (40 columns were a tile of 32
-// and one of 8), 284 us in this form (2.8 TB/s of gathered rows).
+// and one of 8), 237 us in this form (3.4 TB/s of gathered rows).
 //
 // Layouts: the reference indexes B and C row-major through lead_dim whatever
 // their `major` field says; here row-major is the same, and column-major
@@ -31,7 +31,9 @@
 namespace clsp {
 namespace {
 
-constexpr int kThreads = 256;
+// Two warps a CTA: a CTA's slots come free when its longest row is done, and row
+// lengths differ widely (284 us with 256 threads on the matrix above, 237 with 64).
+constexpr int kThreads = 64;
 
 // Element (r, c) of a dense matrix is at r * rs + c * cs.
 struct DenseView {
