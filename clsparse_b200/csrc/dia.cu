@@ -43,12 +43,15 @@
 // r = b and keeps the previous solve's last direction:
 // p = z + (<r,z> / rz_prev) p_prev.
 //
-// Drop-in solves (solver loop mode 3): clsparse{S,D}csrcg and
+// Drop-in solves (solver loop modes 0, 1 and 3): clsparse{S,D}csrcg and
 // clsparse{S,D}csrbicgStab on a banded matrix run as one cooperative launch
 // over a diagonal-storage copy in the solve's own type, in the reference's
 // arithmetic (rows in its CSR-Adaptive order, separately rounded operations),
 // with its stop tests and solver-control bookkeeping (dia_cg_ref_kernel,
 // dia_bicg_ref_kernel below).
+//
+// Solves whose vectors fit in the SMs' registers and shared memory run on chip
+// instead (dia_resident.cu); the kernels here stream theirs through L2.
 //
 // Safety: every barrier wait is bounded (grid_sync.cuh); a timeout leaves
 // the kernel through every CTA and is reported as the barrier-timeout status.
@@ -62,6 +65,8 @@
 
 #include "device_common.cuh"
 #include "dia.h"
+#include "dia_resident.h"
+#include "dia_rows.cuh"
 #include "fused.h"
 #include "grid_sync.cuh"
 #include "internal.h"
@@ -113,18 +118,25 @@ __device__ bool set_insert(int32_t* table, int32_t o) {
 __global__ void dia_offsets_kernel(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ cols, uint32_t n,
                                    int32_t* table, int* flags) {
     __shared__ int32_t st[kSlots];
+    __shared__ int full;  // more offsets than the set holds: nothing left to find
     for (int s = threadIdx.x; s < kSlots; s += blockDim.x) st[s] = kEmpty;
+    if (threadIdx.x == 0) full = 0;
     __syncthreads();
     int bad = 0;
     int32_t last[4] = {kEmpty, kEmpty, kEmpty, kEmpty};  // offsets this thread inserted lately
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        if (*reinterpret_cast<volatile int*>(&full)) break;
         const uint32_t b = rp[i], e = rp[i + 1];
         for (uint32_t k = b; k < e; ++k) {
             const uint32_t c = cols[k];
             if (k > b && c <= cols[k - 1]) bad |= 2;
             const int32_t o = static_cast<int32_t>(static_cast<int64_t>(c) - static_cast<int64_t>(i));
             if (o == last[0] || o == last[1] || o == last[2] || o == last[3]) continue;
-            if (!set_insert(st, o)) bad |= 1;
+            if (!set_insert(st, o)) {
+                bad |= 1;
+                full = 1;
+                break;
+            }
             last[3] = last[2];
             last[2] = last[1];
             last[1] = last[0];
@@ -665,123 +677,6 @@ fail:
 
 // ---- the drop-in CG (clsparse{S,D}csrcg, solver loop mode 3)
 
-// In/out block of one drop-in solve.
-struct DiaCgState {
-    // in: the solver control
-    double rel_tol = 0.0, abs_tol = 0.0;
-    int max_iters = 0;
-    int n_iters_in = 0;  // nIters the control held before the solve (the first stop test sees it)
-    int l2 = 0;          // 0: ||.||_1 stop test as the reference, 1: ||.||_2
-    int stop_nonfinite = 0;
-    // out
-    int n_iters = 0;
-    int zero_b = 0;      // ||b|| == 0: x = b, nothing else done
-    int zero_diag = 0;   // Jacobi with a zero on the main diagonal: nothing written to x
-    int status = 0;      // kStatusCurvature / kStatusNonFinite / kStatusBarrierTimeout
-    double init_res = 0.0, cur_res = 0.0;
-};
-
-// Rows [r0, r1) whose CSR-Adaptive block reduces a row over g > 1 lanes.
-struct LaneRange {
-    uint32_t r0, r1, g;
-};
-constexpr int kMaxLaneRanges = 8;
-
-template <typename T>
-struct DiaCgArgs {
-    using value_type = T;
-    DiaMat<T> A;
-    // CSR arrays of A, for the rows of lane ranges
-    const uint32_t* rp;
-    const uint32_t* cols;
-    const T* vals;
-    LaneRange lanes[kMaxLaneRanges];
-    int nlanes;
-    // A symmetric bit for bit with its offsets symmetric and no padding
-    // diagonals (the kernel's SYM form): the value of lower diagonal d at row
-    // i is read as A[j][i] from its upper partner ND - 1 - d at row
-    // j = i + off[d], and the lower diagonals are not read at all
-    int nd_real;
-    int d0;         // index of the main diagonal (Jacobi)
-    T* invD;        // Jacobi: 1 / a_ii, formed in the prologue; nullptr: no preconditioner
-    const T* b;
-    T* x;           // initial guess in, solution out
-    T* r;
-    T* p[2];        // direction of iteration k in p[k & 1]
-    T* q;           // A p
-    T* z;           // M r (== r without preconditioner)
-    uint32_t n;
-    FusedSync sync;
-    DiaCgState* st;
-};
-
-// Separately rounded products and sums (no contraction into FMAs): the
-// arithmetic of the reference's kernels as compiled for its CPU runs.
-__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
-using dev::mul_rn;
-
-// sum_d A[d][i] * xf(i + off[d]) in T: products rounded, then summed one by
-// one in increasing column order from zero -- the order of a CSR-Adaptive
-// STREAM block that reduces each row on one lane
-// (src/library/kernels/csrmv_adaptive.cl:312-420); the zeros of entries a
-// CSR row does not hold add nothing. Loads are unconditional with
-// out-of-matrix columns clamped and their products zero; a mirrored
-// diagonal's value is read from the upper one at the column's row.
-template <int ND, bool SYM, typename Args, typename XF>
-__device__ __forceinline__ typename Args::value_type dia_row_seq(const Args& a, uint32_t i, XF xf) {
-    using T = typename Args::value_type;
-    const uint32_t n = a.n;
-    T av[ND], xv[ND];
-#pragma unroll
-    for (int d = 0; d < ND; ++d) {
-        const int64_t j = static_cast<int64_t>(i) + a.A.off[d];
-        const bool in = j >= 0 && j < static_cast<int64_t>(n);
-        const uint32_t jc = in ? static_cast<uint32_t>(j) : i;
-        T v;
-        if (SYM && a.A.off[d] < 0)
-            v = __ldg(a.A.vals + static_cast<size_t>(ND - 1 - d) * n + jc);
-        else
-            v = __ldg(a.A.vals + static_cast<size_t>(d) * n + i);
-        const T xj = xf(jc);
-        av[d] = in ? v : T(0);
-        xv[d] = in ? xj : T(0);
-    }
-    T s = T(0);
-#pragma unroll
-    for (int d = 0; d < ND; ++d) s = add_rn(s, mul_rn(av[d], xv[d]));
-    return s;
-}
-
-// Row i of a CSR-Adaptive STREAM block that reduces a row over g lanes (g a
-// power of two): lane l sums the row's products l, l + g, ... one by one,
-// then the lanes combine pairwise at distances g/2, ..., 1. A banded row
-// holds at most kMaxDiags entries, so lanes from kMaxDiags on hold zero.
-template <typename T, typename XF>
-__device__ __noinline__ T csr_row_lanes(const uint32_t* rp, const uint32_t* cols, const T* vals, uint32_t i,
-                                        uint32_t g, XF xf) {
-    T v[kMaxDiags];
-#pragma unroll
-    for (int l = 0; l < kMaxDiags; ++l) v[l] = T(0);
-    g = g > static_cast<uint32_t>(kMaxDiags) ? static_cast<uint32_t>(kMaxDiags) : g;
-    const uint32_t b = rp[i], e = rp[i + 1];
-    for (uint32_t k = b; k < e; ++k) {
-        const uint32_t l = (k - b) & (g - 1);
-        v[l] = add_rn(v[l], mul_rn(__ldg(vals + k), xf(cols[k])));
-    }
-    for (uint32_t off = g / 2; off > 0; off >>= 1)
-        for (uint32_t l = 0; l < off; ++l) v[l] = add_rn(v[l], v[l + off]);
-    return v[0];
-}
-
-// q_i = (A xf)_i in the reference's order for row i.
-template <int ND, bool SYM, typename Args, typename XF>
-__device__ __forceinline__ typename Args::value_type cg_row(const Args& a, uint32_t i, XF xf) {
-    for (int k = 0; k < a.nlanes; ++k)
-        if (i >= a.lanes[k].r0 && i < a.lanes[k].r1) return csr_row_lanes(a.rp, a.cols, a.vals, i, a.lanes[k].g, xf);
-    return dia_row_seq<ND, SYM>(a, i, xf);
-}
-
 // The reference's CG (src/library/solvers/conjugate-gradients.hpp:73-226) as
 // one cooperative launch over a matrix stored by diagonal. Scalars in T as
 // the reference's clsparse::scalar<T>, reductions accumulated in FP64:
@@ -932,33 +827,6 @@ fail:
 }
 
 // ---- the drop-in BiCGStab (clsparse{S,D}csrbicgStab, solver loop mode 3)
-
-template <typename T>
-struct DiaBicgArgs {
-    using value_type = T;
-    DiaMat<T> A;
-    const uint32_t* rp;
-    const uint32_t* cols;
-    const T* vals;
-    LaneRange lanes[kMaxLaneRanges];
-    int nlanes;
-    int nd_real;
-    int d0;
-    T* invD;        // Jacobi: 1 / a_ii, formed in the prologue; nullptr: no preconditioner
-    const T* b;
-    T* x;
-    T* r;
-    T* rs;          // r*
-    T* p[2];        // direction of iteration k in p[k & 1]
-    T* AMp[2];      // A M p_k in AMp[k & 1]
-    T* Mp;          // M p_k (== p_k without preconditioner)
-    T* s;
-    T* Ms;          // M s (== s without preconditioner)
-    T* AMs;
-    uint32_t n;
-    FusedSync sync;
-    DiaCgState* st;
-};
 
 // The reference's BiCGStab (src/library/solvers/biconjugate-gradients-
 // stabilized.hpp:61-266) as one cooperative launch, in the arithmetic and row
@@ -1238,6 +1106,25 @@ clsparseStatus dia_detect(const uint32_t* rp, const uint32_t* cols, uint32_t n, 
     return clsparseSuccess;
 }
 
+bool dia_few_offsets(const uint32_t* rp, const uint32_t* cols, uint32_t n, uint32_t max_row, cudaStream_t s) {
+    if (n == 0 || max_row == 0 || max_row > static_cast<uint32_t>(kMaxDiags)) return false;
+    DeviceBuffer table;
+    if (table.ensure(kSlots * sizeof(int32_t) + 64) != cudaSuccess) {
+        cudaGetLastError();
+        return true;  // (not known: the solve looks)
+    }
+    int32_t* t = static_cast<int32_t*>(table.ptr);
+    int* flags = reinterpret_cast<int*>(t + kSlots);
+    cudaMemsetAsync(t, 0x80, kSlots * sizeof(int32_t), s);
+    cudaMemsetAsync(flags, 0, sizeof(int), s);
+    dia_offsets_kernel<<<std::min<uint32_t>((n + 255) / 256, 1184), 256, 0, s>>>(rp, cols, n, t, flags);
+    int h = 0;
+    if (cudaGetLastError() != cudaSuccess || cudaMemcpyAsync(&h, flags, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
+        return true;
+    return (h & 1) == 0;
+}
+
 template <typename VI, typename VO>
 clsparseStatus dia_build(const uint32_t* rp, const uint32_t* cols, const VI* vals, uint32_t n,
                          const DiaOffsets& offs, int nd_pad, DeviceBuffer& buf, cudaStream_t s, DiaMat<VO>& out) {
@@ -1314,6 +1201,13 @@ void dia_classes(int nda, int ndg, bool learned, int& ca, int& cg) {
 
 namespace {
 
+// CLSPARSE_B200_DIA_RESIDENT=0 keeps the banded solves streaming their vectors
+// through L2 (for comparison).
+bool resident_enabled() {
+    const char* e = std::getenv("CLSPARSE_B200_DIA_RESIDENT");
+    return !(e && e[0] == '0' && e[1] == '\0');
+}
+
 // One inner solve as one cooperative launch.
 // Shared memory of the local-t learned form (t for a CTA's rows and the
 // gt_halo rows after them), or 0 when that form does not apply: an offset of
@@ -1336,7 +1230,10 @@ clsparseStatus dia_persistent_solve(DiaPcgArgs<VA, VG> a, bool learned, DiaWork&
                                     DiaPcgState& st) {
     cudaStream_t s = c->stream;
     const uint32_t max_grid = static_cast<uint32_t>(std::max(1, c->sm_count) * std::max(2, kDiaCtasPerSm));
-    const size_t sync_b = align256(fused_sync_bytes(max_grid));
+    // On chip when the vectors fit (dia_resident.cu), else streamed through L2.
+    ResidentPlan plan;
+    const bool resident = resident_enabled() && resident_pcg_plan<VA, VG>(a, learned, c->sm_count, plan);
+    const size_t sync_b = align256(resident ? word_sync_bytes(plan, a.n, sizeof(float), learned ? 2 : plan.words) : fused_sync_bytes(max_grid));
     if (w.sync.ensure(sync_b + align256(sizeof(DiaPcgState))) != cudaSuccess) {
         cudaGetLastError();
         return clsparseOutOfResources;
@@ -1344,7 +1241,7 @@ clsparseStatus dia_persistent_solve(DiaPcgArgs<VA, VG> a, bool learned, DiaWork&
     char* base = static_cast<char*>(w.sync.ptr);
     DiaPcgState* dst = reinterpret_cast<DiaPcgState*>(base + sync_b);
     st.status = 0;
-    cudaMemsetAsync(base, 0, kFusedSyncHead, s);
+    cudaMemsetAsync(base, 0, resident ? sync_b : kFusedSyncHead, s);
     cudaMemcpyAsync(dst, &st, sizeof(st), cudaMemcpyHostToDevice, s);
     a.sync = fused_sync_at(base);
     // failure-path test switches, as for the CSR persistent engine
@@ -1358,7 +1255,10 @@ clsparseStatus dia_persistent_solve(DiaPcgArgs<VA, VG> a, bool learned, DiaWork&
     uint32_t grid = 0;
     cudaError_t e = cudaErrorInvalidValue;
     const int na = a.A.nd, ng = a.G.nd;
-    if (!learned) {
+    if (resident) {
+        e = launch_pcg_resident<VA, VG>(a, learned, plan,
+                                        word_sync_at(base, plan, a.sync.wait_ns, a.sync.never_release), s);
+    } else if (!learned) {
         if (na == 3) e = dia_launch<VA, VG, 0, 3, 3>(a, sms, s, grid);
         else if (na == 5) e = dia_launch<VA, VG, 0, 5, 3>(a, sms, s, grid);
         else if (na == 7) e = dia_launch<VA, VG, 0, 7, 3>(a, sms, s, grid);
@@ -1390,12 +1290,6 @@ clsparseStatus dia_persistent_solve(DiaPcgArgs<VA, VG> a, bool learned, DiaWork&
 
 }  // namespace
 
-template <typename VA, typename VG>
-clsparseStatus dia_pcg_solve(DiaPcgArgs<VA, VG> a, bool learned, DiaWork& w, clsparseControl c,
-                             DiaPcgState& st) {
-    return dia_persistent_solve<VA, VG>(a, learned, w, c, st);
-}
-
 namespace {
 
 // flag |= 1 when A[i][i + off_l] (diagonal dl, off_l < 0) differs bitwise
@@ -1403,7 +1297,8 @@ namespace {
 template <typename T>
 __global__ void dia_sym_check_kernel(const T* __restrict__ vals, uint32_t n, int dl, int du, int32_t off_l,
                                      int* flag) {
-    using U = std::conditional_t<sizeof(T) == 8, unsigned long long, unsigned int>;
+    using U = std::conditional_t<sizeof(T) == 8, unsigned long long,
+                                 std::conditional_t<sizeof(T) == 4, unsigned int, unsigned short>>;
     bool bad = false;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int64_t j = static_cast<int64_t>(i) + off_l;
@@ -1417,6 +1312,38 @@ __global__ void dia_sym_check_kernel(const T* __restrict__ vals, uint32_t n, int
     }
     if (bad) atomicOr(flag, 1);
 }
+
+}  // namespace
+
+template <typename V>
+clsparseStatus dia_mirrored(const DiaMat<V>& M, const DiaOffsets& offs, uint32_t n, DiaWork& w, cudaStream_t s,
+                            bool& sym) {
+    sym = false;
+    const int nd = offs.nd;
+    if (nd < 2 || nd != M.nd) return clsparseSuccess;
+    for (int d = 0; d < nd; ++d)
+        if (offs.off[d] != -offs.off[nd - 1 - d]) return clsparseSuccess;
+    int* flag = reinterpret_cast<int*>(static_cast<int32_t*>(w.table.ptr) + kSlots) + 1;
+    cudaMemsetAsync(flag, 0, sizeof(int), s);
+    const uint32_t grid = std::min<uint32_t>((n + 255) / 256, 1184);
+    for (int d = 0; offs.off[d] < 0; ++d)
+        dia_sym_check_kernel<V><<<grid, 256, 0, s>>>(M.vals, n, d, nd - 1 - d, offs.off[d], flag);
+    int h = 1;
+    if (cudaGetLastError() != cudaSuccess ||
+        cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
+        return clsparseInvalidKernelExecution;
+    sym = h == 0;
+    return clsparseSuccess;
+}
+
+template <typename VA, typename VG>
+clsparseStatus dia_pcg_solve(DiaPcgArgs<VA, VG> a, bool learned, DiaWork& w, clsparseControl c,
+                             DiaPcgState& st) {
+    return dia_persistent_solve<VA, VG>(a, learned, w, c, st);
+}
+
+namespace {
 
 // Whether the drop-in CG runs its SYM form: A symmetric bit for bit with
 // symmetric offsets (off[d] = -off[nd - 1 - d]), at most 5 diagonals (the
@@ -1441,22 +1368,7 @@ clsparseStatus dia_symmetric(const DiaMat<T>& M, const DiaOffsets& offs, uint32_
     if (mode == 0 || nd_pad > kSymMaxDiags || offs.nd != nd_pad) return clsparseSuccess;
     const size_t working = static_cast<size_t>(nd_pad + 7) * n * sizeof(T);
     if (mode != 1 && (l2_bytes == 0 || 2 * working <= l2_bytes)) return clsparseSuccess;
-    const int nd = offs.nd;
-    for (int d = 0; d < nd; ++d)
-        if (offs.off[d] != -offs.off[nd - 1 - d]) return clsparseSuccess;
-    if (nd < 2) return clsparseSuccess;
-    int* flag = reinterpret_cast<int*>(static_cast<int32_t*>(w.table.ptr) + kSlots) + 1;
-    cudaMemsetAsync(flag, 0, sizeof(int), s);
-    const uint32_t grid = std::min<uint32_t>((n + 255) / 256, 1184);
-    for (int d = 0; offs.off[d] < 0; ++d)
-        dia_sym_check_kernel<T><<<grid, 256, 0, s>>>(M.vals, n, d, nd - 1 - d, offs.off[d], flag);
-    int h = 1;
-    if (cudaGetLastError() != cudaSuccess ||
-        cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
-        return clsparseInvalidKernelExecution;
-    sym = h == 0;
-    return clsparseSuccess;
+    return dia_mirrored<T>(M, offs, n, w, s, sym);
 }
 
 // The cooperative kernel of a drop-in solve for an argument block.
@@ -1500,7 +1412,8 @@ clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     // their lane count. A block of another kind, or more such ranges than
     // kMaxLaneRanges, leaves the solve to the graph engine.
     const auto* meta = static_cast<const matrix_meta*>(A->meta);
-    if (meta == nullptr || meta->h_rowBlocks.size() < meta->num_words || meta->num_words < 2)
+    if (meta == nullptr || meta->h_rowBlocks.size() < meta->num_words || meta->num_words < 2 ||
+        meta->max_row > static_cast<uint32_t>(kMaxDiags) || (c->solver_loop_mode != 3 && !meta->few_offsets))
         return clsparseNotImplemented;
     LaneRange lanes[kMaxLaneRanges];
     int nlanes = 0;
@@ -1539,12 +1452,22 @@ clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     // 512^2 five-point (33 MB) 25.0 vs 34.0 us; 1024^2 five-point (134 MB)
     // 82.6 vs 81.6; 128^3 seven-point (288 MB) 191 vs 161. Larger systems
     // run the graph engine.
-    if (BICG && static_cast<size_t>(ca + 11) * n * sizeof(T) > c->l2_bytes) return clsparseNotImplemented;
+    // On chip when the vectors fit (dia_resident.cu), else streamed through L2.
+    ResidentPlan plan;
+    const bool resident =
+        resident_enabled() && (BICG ? resident_bicg_plan<T>(n, offs, ca, c->sm_count, plan)
+                                    : resident_cg_plan<T>(n, offs, ca, jac, false, c->sm_count, plan));
+    if (BICG && !resident && static_cast<size_t>(ca + 11) * n * sizeof(T) > c->l2_bytes) return clsparseNotImplemented;
     DiaMat<T> M;
     stt = dia_build<T, T>(rp, cols, vals, n, offs, ca, w.A, s, M);
     if (stt != clsparseSuccess) return stt;
     bool sym = false;
-    if (!BICG) {
+    if (!BICG && resident && resident_streams(plan, ca) && plan.words) {
+        // not every diagonal fits: a symmetric A keeps its upper half
+        stt = dia_mirrored<T>(M, offs, n, w, s, sym);
+        if (stt != clsparseSuccess) return stt;
+        if (sym) resident_cg_plan<T>(n, offs, ca, jac, true, c->sm_count, plan);
+    } else if (!BICG && !resident) {
         stt = dia_symmetric<T>(M, offs, n, ca, c->l2_bytes, w, s, sym);
         if (stt != clsparseSuccess) return stt;
     }
@@ -1554,7 +1477,8 @@ clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     const int nvec = BICG ? 11 : 6;
     const size_t vb = align256(static_cast<size_t>(n) * sizeof(T));
     const uint32_t max_grid = static_cast<uint32_t>(std::max(1, c->sm_count) * kDiaCtasPerSm);
-    const size_t sync_b = align256(fused_sync_bytes(max_grid));
+    const size_t sync_b =
+        align256(resident ? word_sync_bytes(plan, n, sizeof(T), BICG ? 2 : plan.words) : fused_sync_bytes(max_grid));
     if (w.vecs.ensure(nvec * vb) != cudaSuccess ||
         w.sync.ensure(sync_b + align256(sizeof(DiaCgState))) != cudaSuccess) {
         cudaGetLastError();
@@ -1602,7 +1526,7 @@ clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     h.l2 = sc->normType & 1;
     h.stop_nonfinite = sc->stopOnNonFinite ? 1 : 0;
     a.st = reinterpret_cast<DiaCgState*>(base + sync_b);
-    cudaMemsetAsync(base, 0, kFusedSyncHead, s);
+    cudaMemsetAsync(base, 0, resident ? sync_b : kFusedSyncHead, s);
     cudaMemcpyAsync(a.st, &h, sizeof(h), cudaMemcpyHostToDevice, s);
     a.sync = fused_sync_at(base);
     // failure-path test switches, as for the other persistent solvers
@@ -1614,7 +1538,13 @@ clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const c
 
     const int sms = c->sm_count;
     cudaError_t e = cudaErrorInvalidValue;
-    if (sym) {
+    if (resident) {
+        const WordSync ws = word_sync_at(base, plan, a.sync.wait_ns, a.sync.never_release);
+        if constexpr (BICG)
+            e = launch_bicg_resident<T>(a, plan, ws, s);
+        else
+            e = launch_cg_resident<T>(a, plan, ws, s);
+    } else if (sym) {
         if constexpr (!BICG) {
             if (ca == 3) e = dropin_launch<T, 3, true>(a, sms, s, max_grid);
             else if (ca == 5) e = dropin_launch<T, 5, true>(a, sms, s, max_grid);
@@ -1695,6 +1625,10 @@ template clsparseStatus dia_compensate_diag<float>(const uint32_t*, const uint32
                                                     DiaMat<float>&, float*, cudaStream_t);
 template clsparseStatus dia_compensate_diag<__nv_bfloat16>(const uint32_t*, const uint32_t*, const double*, uint32_t,
                                                             DiaMat<__nv_bfloat16>&, float*, cudaStream_t);
+template clsparseStatus dia_mirrored<float>(const DiaMat<float>&, const DiaOffsets&, uint32_t, DiaWork&, cudaStream_t,
+                                            bool&);
+template clsparseStatus dia_mirrored<__nv_bfloat16>(const DiaMat<__nv_bfloat16>&, const DiaOffsets&, uint32_t, DiaWork&,
+                                                    cudaStream_t, bool&);
 template clsparseStatus dia_jacobi<float>(const DiaMat<float>&, uint32_t, float*, int*, cudaStream_t);
 template clsparseStatus dia_jacobi<__nv_bfloat16>(const DiaMat<__nv_bfloat16>&, uint32_t, float*, int*,
                                                   cudaStream_t);

@@ -62,6 +62,7 @@ struct DiaPcgArgs {
     float* t;               // scratch (unused by the current schedules)
     float* z;
     uint32_t n;
+    bool sym = false;       // A symmetric bit for bit, offsets symmetric, no padding diagonals
     int gt_diag;            // index of G^T's main diagonal (learned solves)
     uint32_t gt_halo;       // largest column offset of G^T (its offsets are >= 0: G is lower triangular)
     FusedSync sync;
@@ -120,6 +121,12 @@ clsparseStatus dia_compensate_diag(const uint32_t* rp, const uint32_t* cols, con
 // a zero; clsparseInvalidValue without a main diagonal.
 template <typename VA>
 clsparseStatus dia_jacobi(const DiaMat<VA>& A, uint32_t n, float* invD, int* status, cudaStream_t s);
+
+// Whether a DIA copy is symmetric bit for bit with symmetric offsets and no
+// padding diagonals (one check kernel per lower diagonal, one wait).
+template <typename V>
+clsparseStatus dia_mirrored(const DiaMat<V>& M, const DiaOffsets& offs, uint32_t n, DiaWork& w, cudaStream_t s,
+                            bool& sym);
 
 // One inner solve (one cooperative launch); st in/out as above.
 template <typename VA, typename VG>

@@ -307,6 +307,9 @@ clsparseStatus create_meta(clsparseCsrMatrix* csrMatx, clsparseControl control, 
     if (cudaMemsetAsync(meta->d_error, 0, sizeof(int), control->stream) != cudaSuccess ||
         cudaStreamSynchronize(control->stream) != cudaSuccess)
         return clsparseInvalidKernelExecution;
+    meta->few_offsets = dia_few_offsets(dev_ptr<const uint32_t>(csrMatx->row_pointer, csrMatx->off_row_pointer),
+                                        dev_ptr<const uint32_t>(csrMatx->col_indices, csrMatx->off_col_indices),
+                                        static_cast<uint32_t>(csrMatx->num_rows), meta->max_row, control->stream);
     meta->h_word_nnz = std::move(word_nnz);
     csrMatx->meta = meta.release();
     return clsparseSuccess;

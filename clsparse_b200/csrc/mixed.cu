@@ -100,6 +100,7 @@ struct BandedInner {
     float* invD = nullptr;
     float* vec[7] = {};  // r0, r1, p0, p1, q, t, z
     int* status = nullptr;
+    bool sym = false;     // A symmetric bit for bit (asked for the learned factor only)
     bool have_p = false;  // a previous solve left a direction to continue
     int pbuf = 0;
     double rz_prev = 0.0;
@@ -135,6 +136,7 @@ bool setup_banded(BandedInner<V>& bi, const clsparseCsrMatrix* A, const Factor* 
                    dia_build<__nv_bfloat16, __nv_bfloat16>(factor->GT.rp, factor->GT.cols, factor->GT.vals, n, ot,
                                                            cg, dw.GT, s, bi.GT) != clsparseSuccess))
         return false;
+    if (factor && dia_mirrored<V>(bi.A, oa, n, dw, s, bi.sym) != clsparseSuccess) return false;
     const size_t stride = (static_cast<size_t>(n) + 63) & ~size_t(63);
     if (dw.vecs.ensure(9 * stride * sizeof(float) + 256) != cudaSuccess) {
         cudaGetLastError();
@@ -187,6 +189,7 @@ clsparseStatus banded_solve(BandedInner<V>& bi, bool learned, bool jacobi, float
     a.t = bi.vec[5];
     a.z = bi.vec[6];
     a.n = n;
+    a.sym = bi.sym;
     a.gt_diag = 0;
     a.gt_halo = 0;
     for (int d = bi.GT.nd - 1; d >= 0; --d) {  // the first zero offset: the real diagonal, padding comes after

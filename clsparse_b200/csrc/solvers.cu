@@ -834,11 +834,16 @@ clsparseStatus cg_solve(cldenseVector* xv, const clsparseCsrMatrix* A, const cld
     if (stt != clsparseSuccess) return stt;
     DeviceGuard guard(c->device);
     const size_t n = A->num_rows;
-    // Loop mode 3: a banded matrix runs the reference's CG as one cooperative
-    // launch over a diagonal-storage copy (dia.cu); other matrices, and the
-    // options that engine does not carry (history, snapshots, extended
+    // Loop modes 0, 1 and 3: a banded matrix runs the reference's CG as one
+    // cooperative launch over a diagonal-storage copy (dia.cu); other matrices,
+    // and the options that engine does not carry (history, snapshots, extended
     // precision, the refinement's continued solves), stay on the engines below.
-    if (c->solver_loop_mode == 3 && std::is_same_v<V, T> && ws == nullptr && n > 0 && !c->extended_precision &&
+    // Modes 0 and 1 (which give the same iterates) take it because it is faster wherever it applies, per iteration
+    // (FP64, graph engine / banded): 512^2 five-point 17.3 / 6.0 us, 1000^2
+    // 34.0 / 16.5, 64^3 seven-point 18.5 / 8.5, 100^3 45.4 / 29.2, 128^3
+    // (streamed) 75 / 71, and a solve of 3,600 rows 3.0 / 1.05 ms. Matrices with
+    // more column offsets than it keeps are known from their meta.
+    if (c->solver_loop_mode != 2 && std::is_same_v<V, T> && ws == nullptr && n > 0 && !c->extended_precision &&
         sc->history == nullptr && sc->snapshotCount == 0 && dia_enabled()) {
         stt = dia_cg_dropin<T>(xv, A, bv, sc, c);
         if (stt != clsparseNotImplemented) {
@@ -957,8 +962,14 @@ clsparseStatus bicg_solve(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     if (stt != clsparseSuccess) return stt;
     DeviceGuard guard(c->device);
     const size_t n = A->num_rows;
-    // loop mode 3 on a banded matrix: one cooperative launch (see cg_solve)
-    if (c->solver_loop_mode == 3 && std::is_same_v<V, T> && n > 0 && !c->extended_precision &&
+    // loop modes 0, 1 and 3 on a banded matrix: one cooperative launch (see
+    // cg_solve). BiCGStab's iteration count moves by a few with the order of the
+    // dot products' sums, and on the reference's own small runs (up to 400 rows)
+    // the graph engine's order keeps it within the pinned two: modes 0 and 1 take
+    // the banded engine from kBandedBicgRows on (90,000 rows: 31.7 -> 8.8 us an
+    // iteration).
+    constexpr size_t kBandedBicgRows = 2048;
+    if ((c->solver_loop_mode == 3 || (c->solver_loop_mode != 2 && n >= kBandedBicgRows)) && std::is_same_v<V, T> && n > 0 && !c->extended_precision &&
         sc->history == nullptr && dia_enabled()) {
         stt = dia_bicg_dropin<T>(xv, A, bv, sc, c);
         if (stt != clsparseNotImplemented) {

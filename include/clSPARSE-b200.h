@@ -236,21 +236,23 @@ CLSPARSE_EXPORT clsparseStatus
 cldenseDdotNoAlloc(clsparseScalar* r, const cldenseVector* x, const cldenseVector* y,
                    cl_command_queue queue);
 
-/* Solver loop driver: 0 = one CUDA graph per solve with a device-side
- * conditional WHILE node (no host round trip per iteration, the default);
- * 1 = host-enqueued chunks of iterations with a device done flag (same
- * iterates as 0); 2 = CG and factorized PCG as ONE persistent cooperative
- * kernel per solve (grid-wide exchanges between phases; needs a
- * CSR-Adaptive meta, otherwise and for BiCGStab the solve runs as in 0;
- * iterates equal up to reduction order); 3 = clsparse{S,D}csrcg and
+/* Solver loop driver. In modes 0, 1 and 3 clsparse{S,D}csrcg and
  * clsparse{S,D}csrbicgStab on a banded matrix with a CSR-Adaptive meta (at
  * most 16 distinct column offsets j - i, columns strictly increasing per row)
- * as ONE cooperative kernel over a private copy of A stored by diagonal,
+ * run as ONE cooperative kernel over a private copy of A stored by diagonal,
  * rebuilt at every call (the reference's row order and rounding, stop tests,
  * nIters and solver-control bookkeeping; iterates equal up to the order of
- * the dot-product sums); matrices without a meta or not banded, a zero or
- * missing diagonal under Jacobi, residual history or snapshots, extended
- * precision, and BiCGStab systems larger than L2 run as in 0. */
+ * the dot-product sums), with the vectors held on chip where they fit;
+ * BiCGStab in modes 0 and 1 from 2048 rows on. Other matrices (no meta, not
+ * banded), a zero or missing diagonal under Jacobi, residual history or
+ * snapshots, extended precision, and BiCGStab systems larger than L2 run as
+ * 0 = one CUDA graph per solve with a device-side conditional WHILE node (no
+ * host round trip per iteration; the default); 1 = host-enqueued chunks of
+ * iterations with a device done flag (same iterates as 0); 2 = CG and
+ * factorized PCG as ONE persistent cooperative kernel per solve (grid-wide
+ * exchanges between phases; needs a CSR-Adaptive meta, otherwise and for
+ * BiCGStab the solve runs on the graph; iterates equal up to reduction
+ * order); 3 = as 0. */
 CLSPARSE_EXPORT clsparseStatus
 clsparseB200SetSolverLoopMode(clsparseControl control, cl_int mode);
 
