@@ -189,6 +189,7 @@ def cg_profile(iters: int):
     api.setup()
     ctrl = api.Control()
     ctrl.set_solver_loop_mode(1)
+    os.environ["CLSPARSE_B200_DIA"] = "0"  # the graph engine's kernels, not the banded engine's one launch
     A = api.CsrMatrix.from_numpy(*matgen.diffusion2d_grf(1024, corr_len=0.05, sigma=2.0, seed=1005))
     A.create_meta(ctrl)
     n = A.num_rows
@@ -379,6 +380,7 @@ def cg_section(ctrl, with_cpu: bool):
         before the timed solves; training time is reported separately.
     Beside each FP64 Jacobi-CG entry, banded_loop_mode3 times the same
     clsparseDcsrcg call with solver loop mode 3 (the banded drop-in engine).
+    (The default mode runs these matrices on the same engine.)
     Each solve is timed on its second call (the first captures the graph).
     Every solution's error against the FP64 oracle solution is stated
     (error_vs_fp64_oracle, relative 2-norm): C1 against the serial oracle

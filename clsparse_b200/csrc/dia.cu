@@ -675,7 +675,7 @@ fail:
     if (tid == 0) atomicOr(&a.st->status, kStatusBarrierTimeout);
 }
 
-// ---- the drop-in CG (clsparse{S,D}csrcg, solver loop mode 3)
+// ---- the drop-in CG (clsparse{S,D}csrcg), streaming
 
 // The reference's CG (src/library/solvers/conjugate-gradients.hpp:73-226) as
 // one cooperative launch over a matrix stored by diagonal. Scalars in T as
@@ -826,7 +826,7 @@ fail:
     if (threadIdx.x == 0) atomicOr(&a.st->status, kStatusBarrierTimeout);
 }
 
-// ---- the drop-in BiCGStab (clsparse{S,D}csrbicgStab, solver loop mode 3)
+// ---- the drop-in BiCGStab (clsparse{S,D}csrbicgStab), streaming
 
 // The reference's BiCGStab (src/library/solvers/biconjugate-gradients-
 // stabilized.hpp:61-266) as one cooperative launch, in the arithmetic and row

@@ -1,5 +1,5 @@
 // Banded (diagonal-storage) solves -- the inner solves of the mixed-precision
-// refinement and the drop-in CG / BiCGStab of solver loop mode 3: types shared
+// refinement and the drop-in CG / BiCGStab: types shared
 // by dia.cu, mixed.cu and solvers.cu. See dia.cu for the storage and the
 // engine.
 #pragma once
@@ -72,7 +72,7 @@ struct DiaPcgArgs {
 // CLSPARSE_B200_DIA=0 keeps every inner solve on CSR.
 bool dia_enabled();
 
-// The drop-in clsparse{S,D}csrcg on the banded engine (solver loop mode 3):
+// The drop-in clsparse{S,D}csrcg on the banded engine (solver loop modes 0, 1 and 3):
 // the reference's CG (operation order, scalar type T, L1 or L2 stop test,
 // nIters bookkeeping, x as initial guess, x = b for a zero right-hand side)
 // as one cooperative launch for a matrix with at most kMaxDiags distinct
@@ -83,8 +83,7 @@ template <typename T>
 clsparseStatus dia_cg_dropin(cldenseVector* x, const clsparseCsrMatrix* A, const cldenseVector* b,
                              clSParseSolverControl sc, clsparseControl c);
 
-// The drop-in clsparse{S,D}csrbicgStab on the banded engine (solver loop
-// mode 3), with the same rules and fallback as dia_cg_dropin.
+// The drop-in clsparse{S,D}csrbicgStab on the banded engine, with the same rules and fallback as dia_cg_dropin.
 template <typename T>
 clsparseStatus dia_bicg_dropin(cldenseVector* x, const clsparseCsrMatrix* A, const cldenseVector* b,
                                clSParseSolverControl sc, clsparseControl c);

@@ -85,7 +85,7 @@ struct _clsparseControl {
     size_t l2_bytes = 0;
     bool async = false;
     bool extended_precision = false;
-    int solver_loop_mode = 0;       // 0 graph while-loop, 1 host chunks, 2 persistent kernel, 3 banded CG
+    int solver_loop_mode = 0;       // 0 and 3 banded engine or graph while-loop, 1 the same with host chunks, 2 persistent kernel
     cudaEvent_t event = nullptr;    // recorded after each call
     cudaStream_t capture_stream = nullptr;  // private stream used for graph capture
     // Reduction scratch: kMaxReduceCtas doubles x 4 partial slots + a ticket.
@@ -95,7 +95,7 @@ struct _clsparseControl {
     std::unique_ptr<clsp::SolverCache> solver_cache;
     std::unique_ptr<clsp::MixedWork> mixed_work;
     std::unique_ptr<clsp::BatchWork> batch_work;
-    std::unique_ptr<clsp::DiaWork> dia_cg;  // banded drop-in CG (solver loop mode 3)
+    std::unique_ptr<clsp::DiaWork> dia_cg;  // banded drop-in CG / BiCGStab
 };
 
 // CSR-Adaptive meta attached to clsparseCsrMatrix::meta (reference
