@@ -199,3 +199,83 @@ def test_coo_csr_runs(ctrl, dt, rows, nnz, off):
         g = got.cpu().numpy()
         np.testing.assert_array_equal(g[off:off + nnz], ref)
         assert (g[:off] == 55).all() and (g[off + nnz:] == 55).all()
+
+
+def conversions(ctrl, rows, r):
+    """coo2csr and csr2coo of sorted row indices r (FP64) as two closures, and
+    what they write."""
+    nnz = len(r)
+    ri = torch.tensor(np.asarray(r, dtype=np.int32), device="cuda")
+    ci = torch.arange(nnz, dtype=torch.int32, device="cuda") % 777
+    vv = torch.rand(nnz, dtype=torch.float64, device="cuda")
+    cm = coo_struct(ri, ci, vv, rows, 777)
+    out = api.CsrMatrix(*(torch.full((k,), -7, dtype=d, device="cuda") for k, d in
+                          ((rows + 1, torch.int32), (nnz, torch.int32), (nnz, torch.float64))), 777)
+    back = [torch.full_like(a, -5) for a in (ri, ci, vv)]
+    cm2 = coo_struct(*back, 0, 0)
+    to_csr = lambda: api.check(api.lib().clsparseDcoo2csr(C.byref(cm), C.byref(out.s), ctrl.handle), "coo2csr")
+    to_coo = lambda: api.check(api.lib().clsparseDcsr2coo(C.byref(out.s), C.byref(cm2), ctrl.handle), "csr2coo")
+    return to_csr, to_coo, (ri, ci, vv), out, back
+
+
+# gaps between two occupied rows, around a lane's and a warp's share of a gap (16), a chunk of
+# row pointers (32) and a gap CTA's share (32 x 256)
+GAPS = [15, 16, 17, 18, 31, 32, 33, 34, 62, 63, 64, 65, 95, 96, 97, 8191, 8192, 8193, 40000]
+
+
+@pytest.mark.parametrize("first", [0, 1, 31, 32, 200])
+def test_coo_csr_gaps_of_empty_rows(ctrl, first):
+    """Every gap length at every place within a chunk, several within one run
+    of nonzeros, rows with several nonzeros among them, and gaps before and
+    behind: exact."""
+    rows_at = first + np.cumsum([0] + [g for g in GAPS for _ in range(3)])
+    r = np.repeat(rows_at, 1 + np.arange(len(rows_at)) % 3)
+    for tail in (0, 1, 31, 32, 33, 20000):
+        rows = int(r[-1]) + 1 + tail
+        to_csr, to_coo, src, out, back = conversions(ctrl, rows, r)
+        to_csr()
+        want = np.searchsorted(r, np.arange(rows + 1), side="left")
+        np.testing.assert_array_equal(out.row_ptr.cpu().numpy(), want)
+        to_coo()
+        for a, b in zip(src, back):
+            assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("rows_in_run", [8191, 8192, 8193, 8194, 30000, 3000000])
+@pytest.mark.parametrize("nnz", [2, 2048, 2049, 5000])
+def test_csr2coo_runs_among_many_empty_rows(ctrl, rows_in_run, nnz):
+    """A run's rows found by walking the row pointers or by looking its
+    positions up (beyond 8192 rows between its first and last): exact."""
+    r = np.sort(np.concatenate([[0, rows_in_run], np.random.default_rng(nnz).integers(0, rows_in_run + 1, nnz - 2)]))
+    to_csr, to_coo, src, out, back = conversions(ctrl, rows_in_run + 5, r)
+    to_csr()
+    np.testing.assert_array_equal(out.row_ptr.cpu().numpy(), np.searchsorted(r, np.arange(rows_in_run + 6), side="left"))
+    to_coo()
+    for a, b in zip(src, back):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("case", ["spread", "two_blocks", "even"])
+def test_conversions_spread_empty_rows_over_the_device(ctrl, case):
+    """Many empty rows are not left to one CTA: each direction within the time
+    of moving its arrays at a thirtieth of HBM's rate, and 60 us for launches
+    and dependent loads (one CTA took 640 and 6100 us on `spread`, 660 and
+    8700 on `two_blocks`; coo2csr 370 on `even`)."""
+    rng = np.random.default_rng(1)
+    rows, r = {"spread": (10_000_000, np.sort(rng.integers(0, 10_000_000, 3000))),
+               "two_blocks": (10_000_000, np.sort(np.concatenate([rng.integers(0, 50_000, 500_000),
+                                                                  9_950_000 + rng.integers(0, 50_000, 500_000)]))),
+               "even": (1_000_000, np.linspace(0, 999_999, 16_000).astype(np.int64))}[case]
+    to_csr, to_coo, src, out, back = conversions(ctrl, rows, r)
+    bar = 60.0 + (4 * rows + 2 * 16 * len(r)) / 2.0e5  # us; 200 GB/s
+    for fn in (to_csr, to_coo):
+        times = []
+        for _ in range(12):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            fn()
+            e1.record()
+            e1.synchronize()
+            times.append(e0.elapsed_time(e1) * 1e3)
+        assert min(times) <= bar, (times, bar)
+    assert torch.equal(src[0], back[0])
