@@ -1046,13 +1046,17 @@ int dia_grid(int sm_count, size_t smem) {
     return std::max(1, sm_count) * std::max(1, std::min(b, kDiaCtasPerSm));
 }
 
-// smem: dynamic shared memory of the launch (the local-t learned form).
+constexpr size_t kLocalTMaxSmem = 160 * 1024;
+
+// smem: dynamic shared memory of the launch (the local-t learned form). The
+// kernel's limit is set to the most any launch asks for, so that threads with
+// different matrices set the same value.
 template <typename VA, typename VG, int PK, int NDA, int NDG>
 cudaError_t dia_launch(DiaPcgArgs<VA, VG>& a, int sm_count, cudaStream_t s, uint32_t& grid, size_t smem = 0) {
     const void* k = reinterpret_cast<const void*>(dia_pcg_kernel<VA, VG, PK, NDA, NDG>);
     if (smem > 0) {
         const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   static_cast<int>(smem));
+                                                   static_cast<int>(kLocalTMaxSmem));
         if (e != cudaSuccess) return e;
     }
     grid = static_cast<uint32_t>(dia_grid<VA, VG, PK, NDA, NDG>(sm_count, smem));
@@ -1212,7 +1216,6 @@ bool resident_enabled() {
 // Shared memory of the local-t learned form (t for a CTA's rows and the
 // gt_halo rows after them), or 0 when that form does not apply: an offset of
 // G^T below zero, more than kLocalTMaxSmem bytes, or CLSPARSE_B200_DIA_LOCAL_T=0.
-constexpr size_t kLocalTMaxSmem = 160 * 1024;
 template <typename VA, typename VG>
 size_t local_t_smem(const DiaPcgArgs<VA, VG>& a, int sm_count) {
     const char* env = std::getenv("CLSPARSE_B200_DIA_LOCAL_T");

@@ -1004,10 +1004,16 @@ fail:
     if (t == 0) atomicOr(&a.st->status, kStatusBarrierTimeout);
 }
 
+// Dynamic shared memory a resident CTA may use: the 227 KB an SM gives one
+// CTA, less the kernel's static part.
+constexpr size_t kResidentSmem = 232448 - 4096;
+
+// (The attribute belongs to the kernel, not to the launch: always the same
+// value, so that another thread's smaller plan cannot come between.)
 template <typename Args>
 cudaError_t resident_launch(const void* k, Args& args, int threads, cudaStream_t s) {
     const cudaError_t e =
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(args.plan.smem));
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kResidentSmem));
     if (e != cudaSuccess) return e;
     void* p[] = {&args};
     return cudaLaunchCooperativeKernel(k, dim3(args.plan.grid), dim3(threads), p, args.plan.smem, s);
@@ -1035,10 +1041,6 @@ cudaError_t pcg_launch(DiaPcgResidentArgs<VA, VG>& args, cudaStream_t s) {
                               : reinterpret_cast<const void*>(dia_pcg_resident_kernel<VA, VG, NDA, NDG, many, LEARNED>),
         args, kResThreads, s);
 }
-
-// Dynamic shared memory a resident CTA may use: the 227 KB an SM gives one
-// CTA, less the kernel's static part.
-constexpr size_t kResidentSmem = 232448 - 4096;
 
 // Rows per CTA a solve aims at. An exchange costs more the more CTAs take part
 // (each polls every other's words: 0.4 us with 2, 0.9 with 19, 1.5 with 148,

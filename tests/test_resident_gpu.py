@@ -15,6 +15,8 @@ stencils within a CTA, across neighbours, and across several CTAs (the plain
 exchange of z); 3 to 9 diagonals and padded counts."""
 from __future__ import annotations
 
+import threading
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -206,3 +208,36 @@ def test_default_mode_takes_the_banded_engine_with_its_results(ctrl, orc):
             xg, kg = solve(kind, 0, **other)
             assert abs(kg - k0) <= max(3, 0.1 * k0)
             assert np.linalg.norm(xg - x0) <= 1e-6 * np.linalg.norm(x0)
+
+
+def test_threads_with_different_plans(ctrl):
+    """Two threads with a control each on one stream, whose matrices need the
+    same kernel with different amounts of shared memory: every launch is taken
+    (the limit is the kernel's, shared by the threads: set to each launch's own
+    amount, one thread's smaller value came between the other's two calls)."""
+    errors = []
+
+    def work(offs):
+        c = api.Control(stream)
+        try:
+            n = 1500
+            A = api.CsrMatrix.from_numpy(*banded(n, offs))
+            A.create_meta(c)
+            b = torch.ones(n, dtype=torch.float64, device="cuda")
+            x = torch.zeros(n, dtype=torch.float64, device="cuda")
+            for _ in range(1500):
+                sc = api.SolverControl(L.DIAGONAL, 1, 0.0, 0.0)
+                api.solve("cg", x, A, b, sc, c)
+                sc.release()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+        finally:
+            c.release()
+
+    stream = torch.cuda.current_stream()
+    threads = [threading.Thread(target=work, args=(o,)) for o in ([1, 20], [1, 700])]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
