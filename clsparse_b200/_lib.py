@@ -192,6 +192,7 @@ SIGNATURES = {
     "clsparseB200SolverGetInfo": (clsparseStatus, [_V, P(cl_int), P(C.c_double), P(C.c_double)]),
     "clsparseB200SolverGetDeviceStatus": (clsparseStatus, [_V, P(cl_uint)]),
     "clsparseB200SetSolverLoopMode": (clsparseStatus, [_V, cl_int]),
+    "clsparseB200GetSolverEngine": (clsparseStatus, [_V, C.POINTER(cl_int)]),
     "clsparseB200SolverSetNormType": (clsparseStatus, [_V, cl_int]),
     "clsparseDcsrcgMixed": (clsparseStatus, [_D, _M, _D, _V, cl_int, C.c_double, P(clsparseB200MixedInfo), _V]),
     "clsparseDcsrbicgStabMixed": (clsparseStatus, [_D, _M, _D, _V, cl_int, C.c_double, P(clsparseB200MixedInfo), _V]),

@@ -67,6 +67,13 @@ class Control:
     def set_solver_loop_mode(self, mode: int):
         check(lib().clsparseB200SetSolverLoopMode(self.handle, mode), "clsparseB200SetSolverLoopMode")
 
+    def solver_engine(self) -> str:
+        """The engine the last solve ran on: "none", "graph", "chunks",
+        "persistent", "banded" or "banded-on-chip"."""
+        e = L.cl_int()
+        check(lib().clsparseB200GetSolverEngine(self.handle, C.byref(e)), "clsparseB200GetSolverEngine")
+        return ("none", "graph", "chunks", "persistent", "banded", "banded-on-chip")[e.value]
+
     def release(self):
         if self.handle:
             check(lib().clsparseReleaseControl(self.handle), "clsparseReleaseControl")

@@ -61,6 +61,11 @@ clsparseStatus finish_call(clsparseControl control) {
     return clsparseSuccess;
 }
 
+bool test_fail(const char* step) {
+    const char* e = std::getenv("CLSPARSE_B200_TEST_FAIL");
+    return e != nullptr && std::strstr(e, step) != nullptr;
+}
+
 }  // namespace clsp
 
 void _solverControl::printSummary(clsparseStatus status) const {
@@ -215,6 +220,13 @@ clsparseStatus clsparseB200SetSolverLoopMode(clsparseControl control, cl_int mod
     if (control == nullptr) return clsparseInvalidControlObject;
     if (mode < 0 || mode > 3) return clsparseInvalidValue;
     control->solver_loop_mode = mode;
+    return clsparseSuccess;
+}
+
+clsparseStatus clsparseB200GetSolverEngine(clsparseControl control, cl_int* engine) {
+    if (control == nullptr) return clsparseInvalidControlObject;
+    if (engine == nullptr) return clsparseInvalidValue;
+    *engine = control->engine;
     return clsparseSuccess;
 }
 

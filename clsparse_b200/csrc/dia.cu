@@ -1399,12 +1399,150 @@ cudaError_t dropin_launch(Args& a, int sm_count, cudaStream_t s, uint32_t max_gr
     return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kDiaThreads), args, 0, s);
 }
 
+// One drop-in solve on chip (plan given) or streaming its vectors through L2
+// (sym: the form that reads the lower diagonals from the upper ones). refused:
+// its memory could not be had or its launch was not taken, and nothing ran.
+template <typename T, bool BICG>
+clsparseStatus dropin_run(cldenseVector* xv, const clsparseCsrMatrix* A, const cldenseVector* bv, const DiaMat<T>& M,
+                          const DiaOffsets& offs, const LaneRange* lanes, int nlanes, const ResidentPlan* plan,
+                          bool sym, clSParseSolverControl sc, clsparseControl c, DiaWork& w, bool& refused) {
+    using Args = std::conditional_t<BICG, DiaBicgArgs<T>, DiaCgArgs<T>>;
+    const uint32_t n = static_cast<uint32_t>(A->num_rows);
+    const bool jac = sc->preconditioner == DIAGONAL;
+    const bool resident = plan != nullptr;
+    const int ca = M.nd;
+    cudaStream_t s = c->stream;
+    refused = true;
+    // work vectors -- CG: invD, r, p[0], p[1], q, z; BiCGStab: invD, r, r*,
+    // p[0], p[1], AMp[0], AMp[1], Mp, s, Ms, AMs. On chip: D^-1 where neither
+    // the registers nor the shared memory hold it, and the plain halo vector.
+    const bool inv_global = resident && plan->inv_global, z_global = resident && !BICG && !plan->words;
+    const int nvec = resident ? (inv_global ? 1 : 0) + (z_global ? 1 : 0) : (BICG ? 11 : 6);
+    const size_t vb = align256(static_cast<size_t>(n) * sizeof(T));
+    const uint32_t max_grid = static_cast<uint32_t>(std::max(1, c->sm_count) * kDiaCtasPerSm);
+    const size_t sync_b =
+        align256(resident ? word_sync_bytes(*plan, n, sizeof(T), BICG ? 2 : plan->words) : fused_sync_bytes(max_grid));
+    if (test_fail(resident ? "onchip-alloc" : "banded-alloc") ||
+        (nvec > 0 && w.vecs.ensure(nvec * vb) != cudaSuccess) ||
+        w.sync.ensure(sync_b + align256(sizeof(DiaCgState))) != cudaSuccess) {
+        cudaGetLastError();
+        return clsparseOutOfResources;
+    }
+    char* vbase = static_cast<char*>(w.vecs.ptr);
+    char* base = static_cast<char*>(w.sync.ptr);
+    auto vec = [&](int k) { return reinterpret_cast<T*>(vbase + static_cast<size_t>(k) * vb); };
+    Args a{};
+    a.A = M;
+    a.rp = dev_ptr<const uint32_t>(A->row_pointer, A->off_row_pointer);
+    a.cols = dev_ptr<const uint32_t>(A->col_indices, A->off_col_indices);
+    a.vals = dev_ptr<const T>(A->values, A->off_values);
+    for (int k = 0; k < nlanes; ++k) a.lanes[k] = lanes[k];
+    a.nlanes = nlanes;
+    a.nd_real = offs.nd;
+    a.d0 = main_diag_index(M);
+    a.b = dev_ptr<const T>(bv->values, bv->off_values);
+    a.x = dev_ptr<T>(xv->values, xv->off_values);
+    a.n = n;
+    if (resident) {
+        // (without a vector of its own invD only says that there is a preconditioner)
+        a.invD = !jac ? nullptr : inv_global ? vec(0) : reinterpret_cast<T*>(base);
+        if constexpr (!BICG) a.z = z_global ? vec(inv_global ? 1 : 0) : nullptr;
+    } else {
+        a.invD = jac ? vec(0) : nullptr;
+        a.r = vec(1);
+        if constexpr (BICG) {
+            a.rs = vec(2);
+            a.p[0] = vec(3);
+            a.p[1] = vec(4);
+            a.AMp[0] = vec(5);
+            a.AMp[1] = vec(6);
+            a.Mp = vec(7);
+            a.s = vec(8);
+            a.Ms = jac ? vec(9) : a.s;
+            a.AMs = vec(10);
+        } else {
+            a.p[0] = vec(2);
+            a.p[1] = vec(3);
+            a.q = vec(4);
+            a.z = jac ? vec(5) : a.r;
+        }
+    }
+
+    DiaCgState h;
+    h.rel_tol = sc->relativeTolerance;
+    h.abs_tol = sc->absoluteTolerance;
+    h.max_iters = sc->maxIters;
+    h.n_iters_in = sc->nIters;
+    h.l2 = sc->normType & 1;
+    h.stop_nonfinite = sc->stopOnNonFinite ? 1 : 0;
+    a.st = reinterpret_cast<DiaCgState*>(base + sync_b);
+    cudaMemsetAsync(base, 0, resident ? sync_b : kFusedSyncHead, s);
+    cudaMemcpyAsync(a.st, &h, sizeof(h), cudaMemcpyHostToDevice, s);
+    a.sync = fused_sync_at(base);
+    // failure-path test switches, as for the other persistent solvers
+    if (const char* e = std::getenv("CLSPARSE_B200_BARRIER_WAIT_NS")) {
+        const unsigned long long v = std::strtoull(e, nullptr, 10);
+        if (v > 0) a.sync.wait_ns = v;
+    }
+    if (const char* e = std::getenv("CLSPARSE_B200_TEST_BARRIER_NEVER_RELEASE")) a.sync.never_release = std::atoi(e) != 0;
+
+    const int sms = c->sm_count;
+    cudaError_t e = cudaErrorInvalidValue;
+    if (test_fail(resident ? "onchip-launch" : "banded-launch")) {
+        e = cudaErrorLaunchOutOfResources;
+    } else if (resident) {
+        const WordSync ws = word_sync_at(base, *plan, a.sync.wait_ns, a.sync.never_release);
+        if constexpr (BICG)
+            e = launch_bicg_resident<T>(a, *plan, ws, s);
+        else
+            e = launch_cg_resident<T>(a, *plan, ws, s);
+    } else if (sym) {
+        if constexpr (!BICG) {
+            if (ca == 3) e = dropin_launch<T, 3, true>(a, sms, s, max_grid);
+            else if (ca == 5) e = dropin_launch<T, 5, true>(a, sms, s, max_grid);
+        }
+    } else {
+        if (ca == 3) e = dropin_launch<T, 3, false>(a, sms, s, max_grid);
+        else if (ca == 5) e = dropin_launch<T, 5, false>(a, sms, s, max_grid);
+        else if (ca == 7) e = dropin_launch<T, 7, false>(a, sms, s, max_grid);
+        else if (ca == 9) e = dropin_launch<T, 9, false>(a, sms, s, max_grid);
+        else if (ca == kMaxDiags) e = dropin_launch<T, kMaxDiags, false>(a, sms, s, max_grid);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return clsparseInvalidKernelExecution;
+    }
+    refused = false;
+    c->engine = resident ? kEngineBandedOnChip : kEngineBanded;
+    if (cudaMemcpyAsync(&h, a.st, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess)
+        return clsparseInvalidKernelExecution;
+    if (c->event) cudaEventRecord(c->event, s);
+    sc->deviceStatus = static_cast<cl_uint>(h.status);
+    sc->historyLength = 0;
+    if (h.status & kStatusBarrierTimeout) return clsparseInvalidKernelExecution;
+    if (h.zero_diag) return clsparseNotImplemented;  // x untouched; the graph engine reports the zero
+    if (h.zero_b) {
+        // conjugate-gradients.hpp:87-95 (biconjugate-gradients-stabilized.hpp
+        // alike) resets the tolerances of the control
+        sc->nIters = 0;
+        sc->absoluteTolerance = 0.0;
+        sc->relativeTolerance = 0.0;
+        return clsparseSuccess;
+    }
+    sc->initialResidual = h.init_res;
+    sc->currentResidual = h.cur_res;
+    sc->nIters = h.n_iters;
+    return clsparseSuccess;
+}
+
 // The drop-in solves (clsparse{S,D}csrcg with BICG false, clsparse{S,D}csrbicgStab
-// with BICG true) on the banded engine.
+// with BICG true) on the banded engine: on chip, or streaming where that does not
+// fit or is refused, or clsparseNotImplemented (x untouched) for the graph
+// engine, which needs neither a copy of A nor every SM at once.
 template <typename T, bool BICG>
 clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const cldenseVector* bv,
                           clSParseSolverControl sc, clsparseControl c) {
-    using Args = std::conditional_t<BICG, DiaBicgArgs<T>, DiaCgArgs<T>>;
     const uint32_t n = static_cast<uint32_t>(A->num_rows);
     const uint32_t nnz = static_cast<uint32_t>(A->num_nonzeros);
     if (n == 0 || nnz == 0) return clsparseNotImplemented;
@@ -1441,7 +1579,7 @@ clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     const T* vals = dev_ptr<const T>(A->values, A->off_values);
     DiaOffsets offs;
     clsparseStatus stt = dia_detect(rp, cols, n, nnz, w, s, offs);
-    if (stt == clsparseInvalidValue) return clsparseNotImplemented;  // not banded
+    if (stt == clsparseInvalidValue || stt == clsparseOutOfResources) return clsparseNotImplemented;
     if (stt != clsparseSuccess) return stt;
     int ca = 0, cg = 0;
     dia_classes(offs.nd, 0, false, ca, cg);
@@ -1460,129 +1598,34 @@ clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     const bool resident =
         resident_enabled() && (BICG ? resident_bicg_plan<T>(n, offs, ca, c->sm_count, plan)
                                     : resident_cg_plan<T>(n, offs, ca, jac, false, c->sm_count, plan));
-    if (BICG && !resident && static_cast<size_t>(ca + 11) * n * sizeof(T) > c->l2_bytes) return clsparseNotImplemented;
+    const bool streams = !BICG || static_cast<size_t>(ca + 11) * n * sizeof(T) <= c->l2_bytes;
+    if (!resident && !streams) return clsparseNotImplemented;
     DiaMat<T> M;
-    stt = dia_build<T, T>(rp, cols, vals, n, offs, ca, w.A, s, M);
-    if (stt != clsparseSuccess) return stt;
-    bool sym = false;
-    if (!BICG && resident && resident_streams(plan, ca) && plan.words) {
-        // not every diagonal fits: a symmetric A keeps its upper half
-        stt = dia_mirrored<T>(M, offs, n, w, s, sym);
-        if (stt != clsparseSuccess) return stt;
-        if (sym) resident_cg_plan<T>(n, offs, ca, jac, true, c->sm_count, plan);
-    } else if (!BICG && !resident) {
-        stt = dia_symmetric<T>(M, offs, n, ca, c->l2_bytes, w, s, sym);
-        if (stt != clsparseSuccess) return stt;
-    }
-
-    // work vectors -- CG: invD, r, p[0], p[1], q, z; BiCGStab: invD, r, r*,
-    // p[0], p[1], AMp[0], AMp[1], Mp, s, Ms, AMs
-    const int nvec = BICG ? 11 : 6;
-    const size_t vb = align256(static_cast<size_t>(n) * sizeof(T));
-    const uint32_t max_grid = static_cast<uint32_t>(std::max(1, c->sm_count) * kDiaCtasPerSm);
-    const size_t sync_b =
-        align256(resident ? word_sync_bytes(plan, n, sizeof(T), BICG ? 2 : plan.words) : fused_sync_bytes(max_grid));
-    if (w.vecs.ensure(nvec * vb) != cudaSuccess ||
-        w.sync.ensure(sync_b + align256(sizeof(DiaCgState))) != cudaSuccess) {
-        cudaGetLastError();
-        return clsparseOutOfResources;
-    }
-    char* vbase = static_cast<char*>(w.vecs.ptr);
-    auto vec = [&](int k) { return reinterpret_cast<T*>(vbase + static_cast<size_t>(k) * vb); };
-    Args a{};
-    a.A = M;
-    a.rp = rp;
-    a.cols = cols;
-    a.vals = vals;
-    for (int k = 0; k < nlanes; ++k) a.lanes[k] = lanes[k];
-    a.nlanes = nlanes;
-    a.nd_real = offs.nd;
-    a.d0 = main_diag_index(M);
-    a.invD = jac ? vec(0) : nullptr;
-    a.b = dev_ptr<const T>(bv->values, bv->off_values);
-    a.x = dev_ptr<T>(xv->values, xv->off_values);
-    a.r = vec(1);
-    a.n = n;
-    if constexpr (BICG) {
-        a.rs = vec(2);
-        a.p[0] = vec(3);
-        a.p[1] = vec(4);
-        a.AMp[0] = vec(5);
-        a.AMp[1] = vec(6);
-        a.Mp = vec(7);
-        a.s = vec(8);
-        a.Ms = jac ? vec(9) : a.s;
-        a.AMs = vec(10);
-    } else {
-        a.p[0] = vec(2);
-        a.p[1] = vec(3);
-        a.q = vec(4);
-        a.z = jac ? vec(5) : a.r;
-    }
-
-    char* base = static_cast<char*>(w.sync.ptr);
-    DiaCgState h;
-    h.rel_tol = sc->relativeTolerance;
-    h.abs_tol = sc->absoluteTolerance;
-    h.max_iters = sc->maxIters;
-    h.n_iters_in = sc->nIters;
-    h.l2 = sc->normType & 1;
-    h.stop_nonfinite = sc->stopOnNonFinite ? 1 : 0;
-    a.st = reinterpret_cast<DiaCgState*>(base + sync_b);
-    cudaMemsetAsync(base, 0, resident ? sync_b : kFusedSyncHead, s);
-    cudaMemcpyAsync(a.st, &h, sizeof(h), cudaMemcpyHostToDevice, s);
-    a.sync = fused_sync_at(base);
-    // failure-path test switches, as for the other persistent solvers
-    if (const char* e = std::getenv("CLSPARSE_B200_BARRIER_WAIT_NS")) {
-        const unsigned long long v = std::strtoull(e, nullptr, 10);
-        if (v > 0) a.sync.wait_ns = v;
-    }
-    if (const char* e = std::getenv("CLSPARSE_B200_TEST_BARRIER_NEVER_RELEASE")) a.sync.never_release = std::atoi(e) != 0;
-
-    const int sms = c->sm_count;
-    cudaError_t e = cudaErrorInvalidValue;
-    if (resident) {
-        const WordSync ws = word_sync_at(base, plan, a.sync.wait_ns, a.sync.never_release);
-        if constexpr (BICG)
-            e = launch_bicg_resident<T>(a, plan, ws, s);
-        else
-            e = launch_cg_resident<T>(a, plan, ws, s);
-    } else if (sym) {
-        if constexpr (!BICG) {
-            if (ca == 3) e = dropin_launch<T, 3, true>(a, sms, s, max_grid);
-            else if (ca == 5) e = dropin_launch<T, 5, true>(a, sms, s, max_grid);
+    stt = test_fail("banded-copy") ? clsparseOutOfResources : dia_build<T, T>(rp, cols, vals, n, offs, ca, w.A, s, M);
+    if (stt != clsparseSuccess && stt != clsparseOutOfResources) return stt;
+    const bool copied = stt == clsparseSuccess;
+    bool refused = true;
+    if (copied && resident) {
+        bool sym = false;
+        if (!BICG && resident_streams(plan, ca) && plan.words) {
+            // not every diagonal fits: a symmetric A keeps its upper half
+            stt = dia_mirrored<T>(M, offs, n, w, s, sym);
+            if (stt != clsparseSuccess) return stt;
+            if (sym) resident_cg_plan<T>(n, offs, ca, jac, true, c->sm_count, plan);
         }
-    } else {
-        if (ca == 3) e = dropin_launch<T, 3, false>(a, sms, s, max_grid);
-        else if (ca == 5) e = dropin_launch<T, 5, false>(a, sms, s, max_grid);
-        else if (ca == 7) e = dropin_launch<T, 7, false>(a, sms, s, max_grid);
-        else if (ca == 9) e = dropin_launch<T, 9, false>(a, sms, s, max_grid);
-        else if (ca == kMaxDiags) e = dropin_launch<T, kMaxDiags, false>(a, sms, s, max_grid);
+        stt = dropin_run<T, BICG>(xv, A, bv, M, offs, lanes, nlanes, &plan, false, sc, c, w, refused);
     }
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return clsparseInvalidKernelExecution;
+    if (copied && refused && streams) {
+        bool sym = false;
+        if (!BICG) {
+            stt = dia_symmetric<T>(M, offs, n, ca, c->l2_bytes, w, s, sym);
+            if (stt != clsparseSuccess) return stt;
+        }
+        stt = dropin_run<T, BICG>(xv, A, bv, M, offs, lanes, nlanes, nullptr, sym, sc, c, w, refused);
     }
-    if (cudaMemcpyAsync(&h, a.st, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
-        return clsparseInvalidKernelExecution;
-    if (c->event) cudaEventRecord(c->event, s);
-    sc->deviceStatus = static_cast<cl_uint>(h.status);
-    sc->historyLength = 0;
-    if (h.status & kStatusBarrierTimeout) return clsparseInvalidKernelExecution;
-    if (h.zero_diag) return clsparseNotImplemented;  // x untouched; the graph engine reports the zero
-    if (h.zero_b) {
-        // conjugate-gradients.hpp:87-95 (biconjugate-gradients-stabilized.hpp
-        // alike) resets the tolerances of the control
-        sc->nIters = 0;
-        sc->absoluteTolerance = 0.0;
-        sc->relativeTolerance = 0.0;
-        return clsparseSuccess;
-    }
-    sc->initialResidual = h.init_res;
-    sc->currentResidual = h.cur_res;
-    sc->nIters = h.n_iters;
-    return clsparseSuccess;
+    if (!refused) return stt;
+    c->dia_cg.reset();  // its memory is for the graph engine now
+    return clsparseNotImplemented;
 }
 
 }  // namespace

@@ -1106,7 +1106,10 @@ bool resident_cg_plan(uint32_t n, const DiaOffsets& offs, int nd_pad, bool jacob
     SmemBudget b;
     if (!b.take(static_cast<uint64_t>(p.lo) + p.mcap + p.hi, sizeof(T))) return false;
     const bool regs = p.rows <= kFewRows ? inv_in_regs<T, kFewRows>() : inv_in_regs<T, kManyRows>();
-    if (jacobi && !regs && b.take(p.mcap, sizeof(T))) p.inv_smem = 1;  // (read twice an iteration)
+    if (jacobi && !regs) {
+        p.inv_smem = b.take(p.mcap, sizeof(T)) ? 1 : 0;  // (read twice an iteration)
+        p.inv_global = 1 - p.inv_smem;
+    }
     keep_plan(offs.off, nd_pad, sym, sizeof(T), b, p);
     p.smem = b.used();
     return true;

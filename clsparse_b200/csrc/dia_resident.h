@@ -33,6 +33,7 @@ struct ResidentPlan {
     uint32_t grid = 0;         // CTAs, one per SM
     int rows = 0;              // rows per thread the kernel is built for
     int inv_smem = 0;          // D^-1 in shared memory
+    int inv_global = 0;        // D^-1 in a vector of its own
     int words = 0;             // the halo's z as tagged words (else a plain vector)
     uint32_t lo_g = 0, hi_g = 0;  // learned factor: rows G reaches below, G^T above
     // Diagonal d kept in shared memory: row i of the CTA at value at[d] + i of

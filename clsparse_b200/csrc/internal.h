@@ -32,6 +32,21 @@ constexpr uint32_t kBlkSize = 1024;
 constexpr uint32_t kBlockMultiplier = 3;
 constexpr uint32_t kRowsForVector = 1;
 
+// Engine a solve ran on (clsparseB200GetSolverEngine, include/clSPARSE-b200.h).
+enum SolverEngine : int {
+    kEngineNone = 0,
+    kEngineGraph = 1,
+    kEngineChunks = 2,
+    kEnginePersistent = 3,
+    kEngineBanded = 4,
+    kEngineBandedOnChip = 5,
+};
+
+// Failure-path test switch: whether CLSPARSE_B200_TEST_FAIL (a list of step
+// names) asks for this host-side step -- an allocation or a launch -- to
+// report failure without being tried.
+bool test_fail(const char* step);
+
 // A grow-only device allocation.
 struct DeviceBuffer {
     void* ptr = nullptr;
@@ -86,6 +101,7 @@ struct _clsparseControl {
     bool async = false;
     bool extended_precision = false;
     int solver_loop_mode = 0;       // 0 and 3 banded engine or graph while-loop, 1 the same with host chunks, 2 persistent kernel
+    int engine = clsp::kEngineNone; // what the last solve ran on (a SolverEngine)
     cudaEvent_t event = nullptr;    // recorded after each call
     cudaStream_t capture_stream = nullptr;  // private stream used for graph capture
     // Reduction scratch: kMaxReduceCtas doubles x 4 partial slots + a ticket.

@@ -557,6 +557,7 @@ template <typename Pro, typename Body, typename Epi>
 clsparseStatus run_solve(clsparseControl c, SolverCache& cache, bool rebuild, const int* d_done,
                          int max_iters, Pro prologue, Body body, Epi epilogue) {
     cudaStream_t s = c->stream;
+    c->engine = c->solver_loop_mode != 1 ? kEngineGraph : kEngineChunks;
     if (c->solver_loop_mode != 1) {
         if (rebuild || cache.exec == nullptr) {
             cache.drop_graph();
@@ -730,12 +731,13 @@ clsparseStatus prepare_cache(clsparseControl c, SolverCache& cache, const Solver
     // [tickets: kTicketBytes][partials]: the SpMV epilogue's two-level
     // reduction needs 2 x (CTAs + 256) partials and 257 counters
     const size_t parts_doubles = std::max<size_t>(3 * kMaxReduceCtas, 2 * (static_cast<size_t>(spmv_ctas) + 256));
-    if (cache.vecs.ensure(vec_bytes * nvec + 256) != cudaSuccess ||
-        cache.parts.ensure(parts_doubles * sizeof(double) + kTicketBytes + 256) != cudaSuccess ||
-        cache.state.ensure(sizeof(SolverState<T>) + 256) != cudaSuccess) {
+    while (cache.vecs.ensure(vec_bytes * nvec + 256) != cudaSuccess ||
+           cache.parts.ensure(parts_doubles * sizeof(double) + kTicketBytes + 256) != cudaSuccess ||
+           cache.state.ensure(sizeof(SolverState<T>) + 256) != cudaSuccess) {
         cudaGetLastError();
         cache.valid = false;
-        return clsparseOutOfResources;
+        if (c->dia_cg == nullptr) return clsparseOutOfResources;
+        c->dia_cg.reset();  // what an earlier banded solve keeps, then once more
     }
     if (rebuild) {
         // tickets start at zero; kernels leave them at zero
@@ -769,6 +771,7 @@ void reset_long_row_tickets(const matrix_meta* m, cudaStream_t s) {
 template <typename V, typename T, typename VG>
 clsparseStatus run_fused(clsparseControl c, SolverCache& cache, bool rebuild, FusedCgArgs<V, T, VG>& fa,
                          const CsrView<V>& Av, const CsrView<VG>* G, const CsrView<VG>* Gt, int pk) {
+    c->engine = kEnginePersistent;
     const bool ext = c->extended_precision && pk == 0;
     // all CTAs resident, and no more CTAs than A has row-block words
     const uint32_t words = static_cast<uint32_t>(Av.meta->num_words - 1);

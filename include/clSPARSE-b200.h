@@ -243,7 +243,9 @@ cldenseDdotNoAlloc(clsparseScalar* r, const cldenseVector* x, const cldenseVecto
  * rebuilt at every call (the reference's row order and rounding, stop tests,
  * nIters and solver-control bookkeeping; iterates equal up to the order of
  * the dot-product sums), with the vectors held on chip where they fit;
- * BiCGStab in modes 0 and 1 from 2048 rows on. Other matrices (no meta, not
+ * BiCGStab in modes 0 and 1 from 2048 rows on. That kernel needs every SM of
+ * the device at once and device memory for the copy: where either is refused
+ * the solve runs as below. Other matrices (no meta, not
  * banded), a zero or missing diagonal under Jacobi, residual history or
  * snapshots, extended precision, and BiCGStab systems larger than L2 run as
  * 0 = one CUDA graph per solve with a device-side conditional WHILE node (no
@@ -255,6 +257,13 @@ cldenseDdotNoAlloc(clsparseScalar* r, const cldenseVector* x, const cldenseVecto
  * order); 3 = as 0. */
 CLSPARSE_EXPORT clsparseStatus
 clsparseB200SetSolverLoopMode(clsparseControl control, cl_int mode);
+
+/* Engine the control's last CG or BiCGStab solve ran on (of a mixed-precision
+ * or learned solve: its last inner solve): 0 none yet, 1 CUDA graph, 2
+ * host-enqueued chunks, 3 persistent CSR kernel, 4 banded kernel streaming its
+ * vectors through L2, 5 banded kernel with its vectors on chip. */
+CLSPARSE_EXPORT clsparseStatus
+clsparseB200GetSolverEngine(clsparseControl control, cl_int* engine);
 
 /* Device-resident residual history of the next CG / BiCGStab solves with this
  * solver control (the reference prints these residuals in VERBOSE mode,

@@ -1,0 +1,71 @@
+"""Which engine a CG or BiCGStab solve runs on (clsparseB200GetSolverEngine),
+and that a solve whose banded engine cannot have its memory or its launch runs
+on the next engine instead of failing: on chip, then streaming, then the graph.
+The failures are made on the host (CLSPARSE_B200_TEST_FAIL names the step that
+reports failure without being tried)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import scipy.sparse as sp
+import torch
+
+from clsparse_b200 import _lib as L
+from clsparse_b200 import api, matgen
+
+pytestmark = pytest.mark.gpu
+
+MATS = {"poisson": lambda: matgen.poisson2d(60, 50), "wide3d": lambda: matgen.diffusion((30, 30, 6), np.ones(5400))}
+
+
+def solve(ctrl, kind, mat, mode=0, dtype=torch.float64, meta=True, precond=L.DIAGONAL):
+    ctrl.set_solver_loop_mode(mode)
+    A = api.CsrMatrix.from_numpy(*mat, dtype=dtype)
+    if meta:
+        A.create_meta(ctrl)
+    n = len(mat[0]) - 1
+    b = np.random.default_rng(3).uniform(-1, 1, n)
+    x = torch.zeros(n, dtype=dtype, device="cuda")
+    sc = api.SolverControl(precond, 3000, 1e-9 if dtype == torch.float64 else 1e-4, 0.0)
+    info = api.solve(kind, x, A, torch.tensor(b, dtype=dtype, device="cuda"), sc, ctrl)
+    status = sc.device_status()
+    sc.release()
+    ctrl.set_solver_loop_mode(0)
+    M = sp.csr_matrix((mat[2], mat[1].astype(np.int64), mat[0].astype(np.int64)), shape=(n, n))
+    res = np.abs(b - M @ x.double().cpu().numpy()).sum() / np.abs(b).sum()
+    assert status & ~8 == 0 and res <= (1e-8 if dtype == torch.float64 else 5e-3)
+    return info["nIters"], ctrl.solver_engine()
+
+
+@pytest.mark.parametrize("kind", ["cg", "bicgstab"])
+def test_engine_of_a_solve(ctrl, kind, monkeypatch):
+    mat = MATS["poisson"]()
+    assert ctrl.solver_engine() == "none"
+    for mode in (0, 1, 3):
+        assert solve(ctrl, kind, mat, mode)[1] == "banded-on-chip"
+        assert solve(ctrl, kind, mat, mode, meta=False)[1] == ("chunks" if mode == 1 else "graph")
+    assert solve(ctrl, kind, mat, 2)[1] == ("persistent" if kind == "cg" else "graph")
+    monkeypatch.setenv("CLSPARSE_B200_DIA_RESIDENT", "0")
+    assert solve(ctrl, kind, mat)[1] == "banded"
+    monkeypatch.setenv("CLSPARSE_B200_DIA", "0")
+    assert solve(ctrl, kind, mat)[1] == "graph"
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
+@pytest.mark.parametrize("precond", [L.DIAGONAL, L.NOPRECOND], ids=["jacobi", "none"])
+@pytest.mark.parametrize("mode", [0, 1, 3])
+@pytest.mark.parametrize("mat", sorted(MATS))
+@pytest.mark.parametrize("kind", ["cg", "bicgstab"])
+def test_solve_falls_back_when_the_banded_engine_is_refused(ctrl, monkeypatch, kind, mat, mode, precond, dtype):
+    graph = "chunks" if mode == 1 else "graph"
+    m = MATS[mat]()
+    k, engine = solve(ctrl, kind, m, mode, dtype, precond=precond)
+    assert engine == "banded-on-chip"
+    for steps, want in (("onchip-alloc", "banded"), ("onchip-launch", "banded"), ("onchip-alloc,banded-alloc", graph),
+                        ("onchip-launch,banded-launch", graph), ("banded-copy", graph)):
+        monkeypatch.setenv("CLSPARSE_B200_TEST_FAIL", steps)
+        kf, engine = solve(ctrl, kind, m, mode, dtype, precond=precond)
+        assert engine == want, steps
+        assert abs(kf - k) <= max(8, 0.25 * k)
+    monkeypatch.delenv("CLSPARSE_B200_TEST_FAIL")
+    assert solve(ctrl, kind, m, mode, dtype, precond=precond) == (k, "banded-on-chip")
