@@ -25,14 +25,21 @@ namespace {
 
 constexpr int kThreads = 256;     // elementwise CTAs
 constexpr int kRedThreads = 512;  // reduction CTAs
-constexpr int kUnroll = 4;        // 16-byte vectors of each operand a thread has in flight
+
+// Vectors of each operand a thread has in flight: 16 bytes each, or (W = 1) single
+// elements, where the operands are not aligned alike. (20 M FP32 elements, axpy: 93
+// us element by element with one load of each operand in flight, 41 with eight,
+// 39 as 16-byte vectors.)
+template <int W>
+constexpr int kUnroll = W > 1 ? 4 : 8;
 
 enum class Ew : int { Add, Sub, Mul, Div };
 enum class Red : int { Plus, Abs, Sqr, Dot };
 
 // A run of elements in 16-byte vectors: `head` elements up to the first
 // 16-byte boundary, `vecs` vectors, then the rest. An operand at another
-// distance from its boundary leaves everything to the scalar ends (vecs 0).
+// distance from its boundary leaves everything to the scalar ends (vecs 0; the
+// launches below then take the elements one by one as vectors of one).
 struct Runs {
     size_t head, vecs;
 };
@@ -47,9 +54,9 @@ Runs runs_of(size_t n, const T* a, const T* b, const T* c) {
     return Runs{head, (n - head) * sizeof(T) / 16};
 }
 
-template <typename T>
-struct alignas(16) Vec {
-    static constexpr int W = 16 / sizeof(T);
+template <typename T, int WIDTH>
+struct alignas(WIDTH * sizeof(T)) Vec {
+    static constexpr int W = WIDTH;
     T v[W];
 };
 
@@ -59,32 +66,33 @@ uint32_t grid_of(size_t work, size_t per_cta, size_t cap) {
     return static_cast<uint32_t>(ctas ? ctas : 1);
 }
 
-// r[i] = f(x[i], y[i]) (NX 1: f(x[i], .)): one pass of kUnroll vectors of each
-// operand per thread, all loaded before the first store (r may be x or y).
-// Bound by HBM: 3,000,001 FP64 elements (72 MB) take 11.3 us, 6.4 TB/s, from
-// DRAM either way; the vectors pay where the operands come from L2.
-template <typename T, int NX, typename F>
+// r[i] = f(x[i], y[i]) (NX 1: f(x[i], .)): one pass of kUnroll vectors of W
+// elements of each operand per thread, all loaded before the first store (r may be
+// x or y). Bound by HBM: 3,000,001 FP64 elements (72 MB) take 11.3 us, 6.4
+// TB/s, from DRAM either way; the vectors pay where the operands come from L2.
+template <typename T, int W, int NX, typename F>
 __global__ void __launch_bounds__(kThreads)
     map_kernel(size_t n, Runs runs, T* r, const T* x, const T* y, const T* __restrict__ alpha_p,
                const T* __restrict__ beta_p, F f) {
     const T a = alpha_p ? *alpha_p : T(0);
     const T b = beta_p ? *beta_p : T(0);
-    using V = Vec<T>;
+    using V = Vec<T, W>;
+    constexpr int U = kUnroll<W>;
     const size_t stride = static_cast<size_t>(gridDim.x) * kThreads;
     const size_t tid = static_cast<size_t>(blockIdx.x) * kThreads + threadIdx.x;
     const V* xv = reinterpret_cast<const V*>(x + runs.head);
     const V* yv = reinterpret_cast<const V*>(y + runs.head);
     V* rv = reinterpret_cast<V*>(r + runs.head);
-    for (size_t i0 = tid; i0 < runs.vecs; i0 += stride * kUnroll) {
-        V p[kUnroll], q[kUnroll];
+    for (size_t i0 = tid; i0 < runs.vecs; i0 += stride * U) {
+        V p[U], q[U];
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u)
+        for (int u = 0; u < U; ++u)
             if (i0 + u * stride < runs.vecs) {
                 p[u] = xv[i0 + u * stride];
                 if constexpr (NX == 2) q[u] = yv[i0 + u * stride];
             }
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u)
+        for (int u = 0; u < U; ++u)
             if (i0 + u * stride < runs.vecs) {
                 V o;
 #pragma unroll
@@ -130,10 +138,15 @@ struct EwOp {
 
 template <typename T, int NX, typename F>
 void launch_map(size_t n, T* r, const T* x, const T* y, const T* alpha, const T* beta, F f, clsparseControl c) {
+    constexpr int W = 16 / sizeof(T);
     const Runs runs = runs_of<T>(n, r, x, NX == 2 ? y : nullptr);
-    const size_t work = runs.vecs ? runs.vecs : n;
-    const uint32_t grid = grid_of(work, kThreads * (runs.vecs ? kUnroll : 4), static_cast<size_t>(c->sm_count) * 64);
-    map_kernel<T, NX, F><<<grid, kThreads, 0, c->stream>>>(n, runs, r, x, y, alpha, beta, f);
+    const size_t cap = static_cast<size_t>(c->sm_count) * 64;
+    if (runs.vecs)
+        map_kernel<T, W, NX, F><<<grid_of(runs.vecs, kThreads * kUnroll<W>, cap), kThreads, 0, c->stream>>>(
+            n, runs, r, x, y, alpha, beta, f);
+    else
+        map_kernel<T, 1, NX, F><<<grid_of(n, kThreads * kUnroll<1>, cap), kThreads, 0, c->stream>>>(
+            n, Runs{0, n}, r, x, y, alpha, beta, f);
 }
 
 // Accumulator type of a reduction: double for floating point, 64-bit integer
@@ -153,12 +166,20 @@ struct RedAcc<int> {
 // the 2-norm (24 MB) 10.5 us with 1184 CTAs of scalar loads, 8.9 here, the dot
 // product (48 MB, from DRAM) 12.8 and 12.6; dot, axpy, axpby and 2-norm in a row
 // 43.4 -> 40.4 us.
-template <typename T, Red OP>
-__global__ void __launch_bounds__(kRedThreads, 2)
+// Element by element (W = 1), 20 M elements, operands aligned differently: FP64 82
+// us with one load of each operand in flight on two CTAs per SM, 58 with eight, 57
+// with four on three CTAs; FP32 77, 31 and 48.
+template <typename T, int W>
+constexpr int kRedUnroll = W > 1 || sizeof(T) == 8 ? 4 : 8;
+template <typename T, int W>
+constexpr int kRedCtas = W > 1 || sizeof(T) == 4 ? 2 : 3;
+template <typename T, int W, Red OP>
+__global__ void __launch_bounds__(kRedThreads, kRedCtas<T, W>)
     reduce_kernel(size_t n, Runs runs, const T* __restrict__ x, const T* __restrict__ y, T* out,
                   typename RedAcc<T>::type* partials, uint32_t* ticket) {
     using U = typename RedAcc<T>::type;
-    using V = Vec<T>;
+    using V = Vec<T, W>;
+    constexpr int N = kRedUnroll<T, W>;
     U acc[1] = {U(0)};
     auto add = [&](T xi, T yi) {
         const U v = static_cast<U>(xi);
@@ -171,16 +192,16 @@ __global__ void __launch_bounds__(kRedThreads, 2)
     const size_t tid = static_cast<size_t>(blockIdx.x) * kRedThreads + threadIdx.x;
     const V* xv = reinterpret_cast<const V*>(x + runs.head);
     const V* yv = reinterpret_cast<const V*>(OP == Red::Dot ? y + runs.head : x);
-    for (size_t i0 = tid; i0 < runs.vecs; i0 += stride * kUnroll) {
-        V p[kUnroll], q[kUnroll];
+    for (size_t i0 = tid; i0 < runs.vecs; i0 += stride * N) {
+        V p[N], q[N];
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u)
+        for (int u = 0; u < N; ++u)
             if (i0 + u * stride < runs.vecs) {
                 p[u] = xv[i0 + u * stride];
                 if constexpr (OP == Red::Dot) q[u] = yv[i0 + u * stride];
             }
 #pragma unroll
-        for (int u = 0; u < kUnroll; ++u)
+        for (int u = 0; u < N; ++u)
             if (i0 + u * stride < runs.vecs) {
 #pragma unroll
                 for (int w = 0; w < V::W; ++w) add(p[u].v[w], OP == Red::Dot ? q[u].v[w] : T(0));
@@ -285,10 +306,16 @@ clsparseStatus do_reduce(clsparseScalar* s, const cldenseVector* x, const cldens
     const T* yp = (OP == Red::Dot) ? dev_ptr<const T>(y->values, y->off_values) : nullptr;
     const T* xp = dev_ptr<const T>(x->values, x->off_values);
     const Runs runs = runs_of<T>(n, xp, yp, static_cast<const T*>(nullptr));
-    const size_t cap = std::min<size_t>(static_cast<size_t>(c->sm_count) * 2, kMaxReduceCtas);
-    const uint32_t grid = runs.vecs ? grid_of(runs.vecs, kRedThreads * kUnroll, cap) : grid_of(n, kRedThreads * 8, cap);
-    reduce_kernel<T, OP><<<grid, kRedThreads, 0, c->stream>>>(n, runs, xp, yp, dev_ptr<T>(s->value, s->off_value),
-                                                              partials, ticket);
+    const size_t sms = static_cast<size_t>(c->sm_count);
+    const auto cap = [&](int per_sm) { return std::min<size_t>(sms * per_sm, kMaxReduceCtas); };
+    constexpr int W = 16 / sizeof(T);
+    T* out = dev_ptr<T>(s->value, s->off_value);
+    if (runs.vecs)
+        reduce_kernel<T, W, OP><<<grid_of(runs.vecs, kRedThreads * kRedUnroll<T, W>, cap(kRedCtas<T, W>)), kRedThreads, 0, c->stream>>>(
+            n, runs, xp, yp, out, partials, ticket);
+    else
+        reduce_kernel<T, 1, OP><<<grid_of(n, kRedThreads * kRedUnroll<T, 1>, cap(kRedCtas<T, 1>)), kRedThreads, 0, c->stream>>>(
+            n, Runs{0, n}, xp, yp, out, partials, ticket);
     return finish_call(c);
 }
 

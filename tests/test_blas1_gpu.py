@@ -151,3 +151,37 @@ def test_vector_runs(ctrl, dtype, n, offs):
                                    (f"cldense{p}nrm2", (y,), np.linalg.norm(yd), np.linalg.norm(yd))):
         api.blas1(name, ("s", s), *args, ctrl=ctrl)
         assert abs(float(s) - ref) <= TOL[dtype] * scale + 1e-300, name
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
+@pytest.mark.parametrize("op", ["dot", "axpy"])
+def test_operands_aligned_differently_are_not_much_slower(ctrl, op, dtype):
+    """Operands that start differently off a 16-byte boundary go element by
+    element, with as many bytes in flight: at most 1.35 times the time of
+    aligned ones on 20 million elements (the element-by-element form with one
+    load in flight per thread took 1.5 to 2.6 times as long)."""
+    n = 20_000_000
+    x, y, r = (torch.rand(n + 4, dtype=dtype, device="cuda") for _ in range(3))
+    a, s = t([0.5], dtype), torch.zeros(1, dtype=dtype, device="cuda")
+    p = "D" if dtype == torch.float64 else "S"
+
+    def best(shift):
+        xs, ys, rs = x[:n], y[shift:shift + n], r[:n]
+        times = []
+        for _ in range(12):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(4):
+                if op == "dot":
+                    api.blas1(f"cldense{p}dot", ("s", s), xs, ys, ctrl=ctrl)
+                else:
+                    api.blas1(f"cldense{p}axpy", rs, ("s", a), xs, ys, ctrl=ctrl)
+            e1.record()
+            e1.synchronize()
+            times.append(e0.elapsed_time(e1))
+        return min(times)
+
+    ctrl.enable_async(True)
+    aligned, shifted = best(0), best(1)
+    ctrl.enable_async(False)
+    assert shifted <= 1.35 * aligned, (shifted, aligned)
