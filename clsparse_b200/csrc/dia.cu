@@ -1401,11 +1401,12 @@ cudaError_t dropin_launch(Args& a, int sm_count, cudaStream_t s, uint32_t max_gr
 
 // One drop-in solve on chip (plan given) or streaming its vectors through L2
 // (sym: the form that reads the lower diagonals from the upper ones). refused:
-// its memory could not be had or its launch was not taken, and nothing ran.
+// its memory could not be had or its launch was not taken, and nothing ran; or,
+// in the default loop modes, one of its waits ran out, and x is as it was.
 template <typename T, bool BICG>
 clsparseStatus dropin_run(cldenseVector* xv, const clsparseCsrMatrix* A, const cldenseVector* bv, const DiaMat<T>& M,
                           const DiaOffsets& offs, const LaneRange* lanes, int nlanes, const ResidentPlan* plan,
-                          bool sym, clSParseSolverControl sc, clsparseControl c, DiaWork& w, bool& refused) {
+                          bool sym, clSParseSolverControl sc, clsparseControl c, DiaWork& w, bool& refused, bool& timed_out) {
     using Args = std::conditional_t<BICG, DiaBicgArgs<T>, DiaCgArgs<T>>;
     const uint32_t n = static_cast<uint32_t>(A->num_rows);
     const bool jac = sc->preconditioner == DIAGONAL;
@@ -1417,7 +1418,12 @@ clsparseStatus dropin_run(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     // p[0], p[1], AMp[0], AMp[1], Mp, s, Ms, AMs. On chip: D^-1 where neither
     // the registers nor the shared memory hold it, and the plain halo vector.
     const bool inv_global = resident && plan->inv_global, z_global = resident && !BICG && !plan->words;
-    const int nvec = resident ? (inv_global ? 1 : 0) + (z_global ? 1 : 0) : (BICG ? 11 : 6);
+    const int nwork = resident ? (inv_global ? 1 : 0) + (z_global ? 1 : 0) : (BICG ? 11 : 6);
+    // The default modes have the graph engine, whose kernels wait for nothing,
+    // behind this one: they keep the initial guess for it (2 to 3 us a solve;
+    // loop mode 3 reports the timeout instead).
+    const bool keep_x = c->solver_loop_mode != 3;
+    const int nvec = nwork + (keep_x ? 1 : 0);
     const size_t vb = align256(static_cast<size_t>(n) * sizeof(T));
     const uint32_t max_grid = static_cast<uint32_t>(std::max(1, c->sm_count) * kDiaCtasPerSm);
     const size_t sync_b =
@@ -1478,6 +1484,7 @@ clsparseStatus dropin_run(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     a.st = reinterpret_cast<DiaCgState*>(base + sync_b);
     cudaMemsetAsync(base, 0, resident ? sync_b : kFusedSyncHead, s);
     cudaMemcpyAsync(a.st, &h, sizeof(h), cudaMemcpyHostToDevice, s);
+    if (keep_x) cudaMemcpyAsync(vec(nwork), a.x, n * sizeof(T), cudaMemcpyDeviceToDevice, s);
     a.sync = fused_sync_at(base);
     // failure-path test switches, as for the other persistent solvers
     if (const char* e = std::getenv("CLSPARSE_B200_BARRIER_WAIT_NS")) {
@@ -1517,6 +1524,14 @@ clsparseStatus dropin_run(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     if (cudaMemcpyAsync(&h, a.st, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return clsparseInvalidKernelExecution;
+    if (keep_x && (h.status & kStatusBarrierTimeout)) {
+        refused = true;
+        timed_out = true;
+        if (cudaMemcpyAsync(a.x, vec(nwork), n * sizeof(T), cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess)
+            refused = false;
+        return clsparseInvalidKernelExecution;
+    }
     if (c->event) cudaEventRecord(c->event, s);
     sc->deviceStatus = static_cast<cl_uint>(h.status);
     sc->historyLength = 0;
@@ -1538,7 +1553,7 @@ clsparseStatus dropin_run(cldenseVector* xv, const clsparseCsrMatrix* A, const c
 
 // The drop-in solves (clsparse{S,D}csrcg with BICG false, clsparse{S,D}csrbicgStab
 // with BICG true) on the banded engine: on chip, or streaming where that does not
-// fit or is refused, or clsparseNotImplemented (x untouched) for the graph
+// fit or is refused, or clsparseNotImplemented (x as it was) for the graph
 // engine, which needs neither a copy of A nor every SM at once.
 template <typename T, bool BICG>
 clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const cldenseVector* bv,
@@ -1604,7 +1619,7 @@ clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     stt = test_fail("banded-copy") ? clsparseOutOfResources : dia_build<T, T>(rp, cols, vals, n, offs, ca, w.A, s, M);
     if (stt != clsparseSuccess && stt != clsparseOutOfResources) return stt;
     const bool copied = stt == clsparseSuccess;
-    bool refused = true;
+    bool refused = true, timed_out = false;
     if (copied && resident) {
         bool sym = false;
         if (!BICG && resident_streams(plan, ca) && plan.words) {
@@ -1613,15 +1628,15 @@ clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const c
             if (stt != clsparseSuccess) return stt;
             if (sym) resident_cg_plan<T>(n, offs, ca, jac, true, c->sm_count, plan);
         }
-        stt = dropin_run<T, BICG>(xv, A, bv, M, offs, lanes, nlanes, &plan, false, sc, c, w, refused);
+        stt = dropin_run<T, BICG>(xv, A, bv, M, offs, lanes, nlanes, &plan, false, sc, c, w, refused, timed_out);
     }
-    if (copied && refused && streams) {
+    if (copied && refused && !timed_out && streams) {
         bool sym = false;
         if (!BICG) {
             stt = dia_symmetric<T>(M, offs, n, ca, c->l2_bytes, w, s, sym);
             if (stt != clsparseSuccess) return stt;
         }
-        stt = dropin_run<T, BICG>(xv, A, bv, M, offs, lanes, nlanes, nullptr, sym, sc, c, w, refused);
+        stt = dropin_run<T, BICG>(xv, A, bv, M, offs, lanes, nlanes, nullptr, sym, sc, c, w, refused, timed_out);
     }
     if (!refused) return stt;
     c->dia_cg.reset();  // its memory is for the graph engine now

@@ -245,7 +245,9 @@ cldenseDdotNoAlloc(clsparseScalar* r, const cldenseVector* x, const cldenseVecto
  * the dot-product sums), with the vectors held on chip where they fit;
  * BiCGStab in modes 0 and 1 from 2048 rows on. That kernel needs every SM of
  * the device at once and device memory for the copy: where either is refused
- * the solve runs as below. Other matrices (no meta, not
+ * the solve runs as below, as it does in modes 0 and 1 when a wait of the
+ * kernel's CTAs for one another runs out (4 s); mode 3 then returns
+ * clsparseInvalidKernelExecution. Other matrices (no meta, not
  * banded), a zero or missing diagonal under Jacobi, residual history or
  * snapshots, extended precision, and BiCGStab systems larger than L2 run as
  * 0 = one CUDA graph per solve with a device-side conditional WHILE node (no

@@ -69,3 +69,43 @@ def test_solve_falls_back_when_the_banded_engine_is_refused(ctrl, monkeypatch, k
         assert abs(kf - k) <= max(8, 0.25 * k)
     monkeypatch.delenv("CLSPARSE_B200_TEST_FAIL")
     assert solve(ctrl, kind, m, mode, dtype, precond=precond) == (k, "banded-on-chip")
+
+
+@pytest.mark.parametrize("resident", [True, False], ids=["onchip", "streamed"])
+@pytest.mark.parametrize("kind", ["cg", "bicgstab"])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_wait_that_runs_out_in_a_default_mode_is_not_an_error(ctrl, monkeypatch, mode, kind, resident):
+    """With one CTA never releasing its exchange every wait runs out (2 ms):
+    the default modes solve on the graph engine from the same initial guess, bit
+    for bit what that engine alone gives; loop mode 3 reports it (the other
+    tests)."""
+    mat = MATS["poisson"]()
+    n = len(mat[0]) - 1
+    rng = np.random.default_rng(8)
+    b, x0 = (torch.tensor(rng.uniform(-1, 1, n), device="cuda") for _ in range(2))
+    A = api.CsrMatrix.from_numpy(*mat)
+    A.create_meta(ctrl)
+    ctrl.set_solver_loop_mode(mode)
+
+    def run():
+        x = x0.clone()
+        sc = api.SolverControl(L.DIAGONAL, 3000, 1e-9, 0.0)
+        info = api.solve(kind, x, A, b, sc, ctrl)
+        status = sc.device_status()
+        sc.release()
+        return x, info, status
+
+    monkeypatch.setenv("CLSPARSE_B200_DIA", "0")
+    xg, ig, sg = run()
+    monkeypatch.delenv("CLSPARSE_B200_DIA")
+    if not resident:
+        monkeypatch.setenv("CLSPARSE_B200_DIA_RESIDENT", "0")
+    monkeypatch.setenv("CLSPARSE_B200_TEST_BARRIER_NEVER_RELEASE", "1")
+    monkeypatch.setenv("CLSPARSE_B200_BARRIER_WAIT_NS", "2000000")
+    x, i, s = run()
+    assert ctrl.solver_engine() == ("chunks" if mode == 1 else "graph")
+    assert torch.equal(x, xg) and i == ig and s == sg
+    monkeypatch.delenv("CLSPARSE_B200_TEST_BARRIER_NEVER_RELEASE")
+    run()
+    assert ctrl.solver_engine() == ("banded-on-chip" if resident else "banded")
+    ctrl.set_solver_loop_mode(0)
