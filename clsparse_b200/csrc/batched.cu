@@ -527,7 +527,7 @@ clsparseStatus clsparseScsrcgBatched(cldenseVector* x, const clsparseCsrMatrix* 
     cudaStream_t s = control->stream;
 
     const size_t vb = ((n * 4 + 255) / 256) * 256;
-    const size_t meta_bytes = 16 + (nsys + 1) * 4 * 2 + nsys * 4 + nsys + 256;
+    const size_t meta_bytes = 16 + (nsys + 1) * 4 * 2 + nsys * 4 * 2 + nsys + 256;
     const size_t out_bytes = nsys * (4 + 8 + 4) + 64;
     if (w.meta.ensure(meta_bytes) != cudaSuccess ||
         w.out.ensure(out_bytes) != cudaSuccess) {
@@ -539,7 +539,8 @@ clsparseStatus clsparseScsrcgBatched(cldenseVector* x, const clsparseCsrMatrix* 
     uint32_t* d_off = reinterpret_cast<uint32_t*>(mb + 16);
     uint32_t* d_bnd = d_off + (nsys + 1);
     uint32_t* d_order = d_bnd + (nsys + 1);
-    uint8_t* d_lanes = reinterpret_cast<uint8_t*>(d_order + nsys);
+    uint32_t* d_rest = d_order + nsys;  // systems of the general kernel
+    uint8_t* d_lanes = reinterpret_cast<uint8_t*>(d_rest + nsys);
     const uint32_t* rp = dev_ptr<const uint32_t>(A->row_pointer, A->off_row_pointer);
 
     // nonzeros per system from the row pointers at the system boundaries
@@ -635,7 +636,7 @@ clsparseStatus clsparseScsrcgBatched(cldenseVector* x, const clsparseCsrMatrix* 
             if (at[k] >= 0) ctas += static_cast<uint64_t>(sizes[at[k]][1]);
         }
     }
-    std::vector<uint32_t> lists, rest;  // device lists: the classes one after another, then the rest
+    std::vector<uint32_t> lists, rest;  // the classes' systems one after another; the general kernel's
     for (uint32_t k : order) {
         if (at[k] < 0) {
             rest.push_back(k);
@@ -645,9 +646,36 @@ clsparseStatus clsparseScsrcgBatched(cldenseVector* x, const clsparseCsrMatrix* 
         classes[at[k]].smem = std::max(classes[at[k]].smem, place(k, at[k]));
     }
     for (const ResidentClass& c : classes) lists.insert(lists.end(), c.list.begin(), c.list.end());
-    const size_t rest_at = lists.size();
-    lists.insert(lists.end(), rest.begin(), rest.end());
-    cudaMemcpyAsync(d_order, lists.data(), nsys * 4, cudaMemcpyHostToDevice, s);
+    if (!lists.empty()) cudaMemcpyAsync(d_order, lists.data(), lists.size() * 4, cudaMemcpyHostToDevice, s);
+
+    // The general kernel's vectors, and the diagonals of its systems when all
+    // of them are banded; before anything is launched, so that x is untouched when
+    // they cannot be had.
+    std::vector<uint64_t> hbase;
+    uint64_t total = 0;
+    bool banded = false;
+    auto general_memory = [&]() {
+        banded = dia;
+        for (uint32_t k : rest) banded = banded && hnd[k] > 0;
+        total = 0;
+        if (banded) {
+            hbase.assign(nsys, 0);
+            for (uint32_t k : rest) {
+                hbase[k] = total;
+                total += static_cast<uint64_t>(hnd[k]) * (off[k + 1] - off[k]);
+            }
+        }
+        if (!test_fail("batched-alloc") && w.vecs.ensure(4 * vb + 256) == cudaSuccess) {
+            if (banded && w.dia.ensure(total * sizeof(float) + 256) != cudaSuccess) {
+                cudaGetLastError();
+                banded = false;  // (their products from CSR then)
+            }
+            return true;
+        }
+        cudaGetLastError();
+        return false;
+    };
+    if (!rest.empty() && !general_memory()) return clsparseOutOfResources;
 
     char* ob = static_cast<char*>(w.out.ptr);
     double* d_residual = reinterpret_cast<double*>(ob);
@@ -657,9 +685,9 @@ clsparseStatus clsparseScsrcgBatched(cldenseVector* x, const clsparseCsrMatrix* 
     float* xp = dev_ptr<float>(x->values, x->off_values);
     const float* bp = dev_ptr<const float>(b->values, b->off_values);
 
-    bool failed = false;
+    bool failed = false, no_memory = false;
     size_t forked = 0;
-    if (rest_at > 0) {
+    if (!lists.empty()) {
         // each class on a stream of its own, after what the caller's stream holds
         size_t used = 0;
         for (const ResidentClass& c : classes) used += c.list.empty() ? 0 : 1;
@@ -670,73 +698,71 @@ clsparseStatus clsparseScsrcgBatched(cldenseVector* x, const clsparseCsrMatrix* 
         ResidentArgs ra{vals, cols, rp,    xp,      bp,         d_off,       d_order,
                         doffs, dnd, d_iters, d_residual, d_converged, solverControl->maxIters,
                         solverControl->relativeTolerance};
+        std::vector<uint32_t> refused;
         for (const ResidentClass& c : classes) {
             if (c.list.empty()) continue;
             cudaStream_t cs = w.streams[forked];
             failed |= cudaStreamWaitEvent(cs, w.begin, 0) != cudaSuccess;
-            failed |= (c.threads == kResWide ? launch_resident<kResWide>(ra, c, cs)
-                                             : launch_resident<kResSmall>(ra, c, cs)) != cudaSuccess;
+            const cudaError_t e = failed || test_fail("batched-launch") ? cudaErrorLaunchOutOfResources
+                                  : c.threads == kResWide               ? launch_resident<kResWide>(ra, c, cs)
+                                                                        : launch_resident<kResSmall>(ra, c, cs);
+            if (e != cudaSuccess) {
+                cudaGetLastError();
+                refused.insert(refused.end(), c.list.begin(), c.list.end());
+            }
             failed |= cudaEventRecord(w.ends[forked], cs) != cudaSuccess;
             ++forked;
             ra.list += c.list.size();
             if (failed) break;
         }
+        // systems whose launch was not taken: the general kernel's too
+        if (!refused.empty() && !failed) {
+            rest.insert(rest.begin(), refused.begin(), refused.end());
+            no_memory = !general_memory();
+        }
     }
+    failed |= no_memory;
     if (!rest.empty() && !failed) {
         const uint32_t nrest = static_cast<uint32_t>(rest.size());
-        bool banded = dia;
-        for (uint32_t k : rest) banded = banded && hnd[k] > 0;
-        if (w.vecs.ensure(4 * vb + 256) != cudaSuccess) failed = true;
+        cudaMemcpyAsync(d_rest, rest.data(), rest.size() * 4, cudaMemcpyHostToDevice, s);
         BatchArgs a;
         std::memset(&a, 0, sizeof(a));
-        if (banded && !failed) {
-            std::vector<uint64_t> hbase(nsys, 0);
-            uint64_t total = 0;
-            for (uint32_t k : rest) {
-                hbase[k] = total;
-                total += static_cast<uint64_t>(hnd[k]) * (off[k + 1] - off[k]);
-            }
-            if (w.dia.ensure(total * sizeof(float) + 256) != cudaSuccess) {
-                failed = true;
-            } else {
-                cudaMemcpyAsync(dbase, hbase.data(), nsys * 8, cudaMemcpyHostToDevice, s);
-                cudaMemsetAsync(w.dia.ptr, 0, total * sizeof(float), s);
-                batch_dia_fill_kernel<<<nrest, 256, 0, s>>>(rp, cols, vals, d_off, d_order + rest_at, doffs, dnd, dbase,
-                                                            static_cast<float*>(w.dia.ptr));
-                a.dvals = static_cast<const float*>(w.dia.ptr);
-                a.dbase = dbase;
-                a.doffs = doffs;
-                a.dnd = dnd;
-            }
+        if (banded) {
+            cudaMemcpyAsync(dbase, hbase.data(), nsys * 8, cudaMemcpyHostToDevice, s);
+            cudaMemsetAsync(w.dia.ptr, 0, total * sizeof(float), s);
+            batch_dia_fill_kernel<<<nrest, 256, 0, s>>>(rp, cols, vals, d_off, d_rest, doffs, dnd, dbase,
+                                                        static_cast<float*>(w.dia.ptr));
+            a.dvals = static_cast<const float*>(w.dia.ptr);
+            a.dbase = dbase;
+            a.doffs = doffs;
+            a.dnd = dnd;
         }
-        if (!failed) {
-            a.vals = vals;
-            a.cols = cols;
-            a.rp = rp;
-            a.x = xp;
-            a.b = bp;
-            char* vbase = static_cast<char*>(w.vecs.ptr);
-            a.r = reinterpret_cast<float*>(vbase);
-            a.p = reinterpret_cast<float*>(vbase + vb);
-            a.q = reinterpret_cast<float*>(vbase + 2 * vb);
-            a.invd = reinterpret_cast<float*>(vbase + 3 * vb);
-            a.off = d_off;
-            a.order = d_order + rest_at;
-            a.lanes = d_lanes;
-            a.counter = d_counter;
-            a.residual = d_residual;
-            a.iters = d_iters;
-            a.converged = d_converged;
-            a.nsys = nrest;
-            a.max_iters = solverControl->maxIters;
-            a.tol = solverControl->relativeTolerance;
-            int per_sm = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batched_cg_kernel, kThreads, 0);
-            const uint32_t grid = std::min(static_cast<uint32_t>(control->sm_count * std::max(per_sm, 1)), nrest);
-            cudaMemsetAsync(d_counter, 0, 16, s);
-            batched_cg_kernel<<<grid, kThreads, 0, s>>>(a);
-            failed |= cudaGetLastError() != cudaSuccess;
-        }
+        a.vals = vals;
+        a.cols = cols;
+        a.rp = rp;
+        a.x = xp;
+        a.b = bp;
+        char* vbase = static_cast<char*>(w.vecs.ptr);
+        a.r = reinterpret_cast<float*>(vbase);
+        a.p = reinterpret_cast<float*>(vbase + vb);
+        a.q = reinterpret_cast<float*>(vbase + 2 * vb);
+        a.invd = reinterpret_cast<float*>(vbase + 3 * vb);
+        a.off = d_off;
+        a.order = d_rest;
+        a.lanes = d_lanes;
+        a.counter = d_counter;
+        a.residual = d_residual;
+        a.iters = d_iters;
+        a.converged = d_converged;
+        a.nsys = nrest;
+        a.max_iters = solverControl->maxIters;
+        a.tol = solverControl->relativeTolerance;
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batched_cg_kernel, kThreads, 0);
+        const uint32_t grid = std::min(static_cast<uint32_t>(control->sm_count * std::max(per_sm, 1)), nrest);
+        cudaMemsetAsync(d_counter, 0, 16, s);
+        batched_cg_kernel<<<grid, kThreads, 0, s>>>(a);
+        failed |= cudaGetLastError() != cudaSuccess;
     }
     for (size_t k = 0; k < forked; ++k) failed |= cudaStreamWaitEvent(s, w.ends[k], 0) != cudaSuccess;
     if (failed) {
@@ -744,7 +770,7 @@ clsparseStatus clsparseScsrcgBatched(cldenseVector* x, const clsparseCsrMatrix* 
         cudaGetLastError();
         for (size_t k = 0; k < forked; ++k) cudaStreamSynchronize(w.streams[k]);
         cudaStreamSynchronize(s);
-        return clsparseInvalidKernelExecution;
+        return no_memory ? clsparseOutOfResources : clsparseInvalidKernelExecution;
     }
 
     std::vector<double> res(nsys);

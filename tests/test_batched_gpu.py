@@ -175,3 +175,40 @@ def test_resident_sizes_against_csr(ctrl, case, monkeypatch):
             u, v = xs["resident"][k][a:e], xs["csr"][k][a:e]
             assert np.linalg.norm(u - v) <= 1e-3 * np.linalg.norm(v), (s, k)
         assert abs(xs["resident"][2][s] - xs["csr"][2][s]) <= 1e-3 * xs["csr"][2][s] + 1e-6
+
+
+def test_batch_without_memory_leaves_x_and_a_refused_launch_is_solved_anyway(ctrl, monkeypatch):
+    """A batch with systems for the chip and one too large for it. When the
+    general kernel's memory cannot be had the call says so before anything has
+    run: x is as it was. When the on-chip launches are not taken, their systems
+    run in the general kernel. (The failures are made on the host.)"""
+    mats = [_banded_spd(n, o, seed=n) for n, o in ((60000, [1, 240]), (9000, [1, 90]), (500, [1, 22]), (700, [1]))]
+    M = sp.block_diag(mats, format="csr")
+    M.sort_indices()
+    off = np.concatenate([[0], np.cumsum([m.shape[0] for m in mats])]).astype(np.uint32)
+    n = M.shape[0]
+    A = api.CsrMatrix.from_numpy(M.indptr.astype(np.uint32), M.indices.astype(np.uint32), M.data, dtype=torch.float32)
+    rng = np.random.default_rng(5)
+    b, x0 = (torch.tensor(rng.uniform(-1, 1, n).astype(np.float32), device="cuda") for _ in range(2))
+
+    def solve():
+        x = x0.clone()
+        sc = api.SolverControl(L.DIAGONAL, 5000, 1e-6, 0.0)
+        try:
+            return x, api.cg_batched(x, A, b, off, sc, ctrl)
+        except api.ClsparseError as e:
+            return x, e.status
+        finally:
+            sc.release()
+
+    x, out = solve()
+    assert out["converged"] == len(mats)
+    monkeypatch.setenv("CLSPARSE_B200_TEST_FAIL", "batched-alloc")
+    xf, status = solve()
+    assert status == L.clsparseOutOfResources and torch.equal(xf, x0)
+    monkeypatch.setenv("CLSPARSE_B200_TEST_FAIL", "batched-launch")
+    xl, out = solve()
+    assert out["converged"] == len(mats) and out["worst_residual"] <= 1e-6
+    assert float((xl - x).norm()) <= 1e-3 * float(x.norm())
+    monkeypatch.delenv("CLSPARSE_B200_TEST_FAIL")
+    assert torch.equal(solve()[0], x)
