@@ -1212,7 +1212,6 @@ bool resident_enabled() {
     return !(e && e[0] == '0' && e[1] == '\0');
 }
 
-// One inner solve as one cooperative launch.
 // Shared memory of the local-t learned form (t for a CTA's rows and the
 // gt_halo rows after them), or 0 when that form does not apply: an offset of
 // G^T below zero, more than kLocalTMaxSmem bytes, or CLSPARSE_B200_DIA_LOCAL_T=0.
@@ -1228,23 +1227,24 @@ size_t local_t_smem(const DiaPcgArgs<VA, VG>& a, int sm_count) {
     return bytes <= kLocalTMaxSmem ? bytes : 0;
 }
 
+// One inner solve: on chip when the vectors fit (plan given), else streamed
+// through L2. refused: its memory could not be had or its launch was not taken.
 template <typename VA, typename VG>
-clsparseStatus dia_persistent_solve(DiaPcgArgs<VA, VG> a, bool learned, DiaWork& w, clsparseControl c,
-                                    DiaPcgState& st) {
+clsparseStatus dia_persistent_run(DiaPcgArgs<VA, VG> a, bool learned, const ResidentPlan* plan, DiaWork& w,
+                                  clsparseControl c, DiaPcgState& st, bool& refused) {
     cudaStream_t s = c->stream;
+    refused = true;
     const uint32_t max_grid = static_cast<uint32_t>(std::max(1, c->sm_count) * std::max(2, kDiaCtasPerSm));
-    // On chip when the vectors fit (dia_resident.cu), else streamed through L2.
-    ResidentPlan plan;
-    const bool resident = resident_enabled() && resident_pcg_plan<VA, VG>(a, learned, c->sm_count, plan);
-    const size_t sync_b = align256(resident ? word_sync_bytes(plan, a.n, sizeof(float), learned ? 2 : plan.words) : fused_sync_bytes(max_grid));
-    if (w.sync.ensure(sync_b + align256(sizeof(DiaPcgState))) != cudaSuccess) {
+    const size_t sync_b = align256(plan ? word_sync_bytes(*plan, a.n, sizeof(float), learned ? 2 : plan->words)
+                                        : fused_sync_bytes(max_grid));
+    if ((plan && test_fail("onchip-alloc")) || w.sync.ensure(sync_b + align256(sizeof(DiaPcgState))) != cudaSuccess) {
         cudaGetLastError();
         return clsparseOutOfResources;
     }
     char* base = static_cast<char*>(w.sync.ptr);
     DiaPcgState* dst = reinterpret_cast<DiaPcgState*>(base + sync_b);
     st.status = 0;
-    cudaMemsetAsync(base, 0, resident ? sync_b : kFusedSyncHead, s);
+    cudaMemsetAsync(base, 0, plan ? sync_b : kFusedSyncHead, s);
     cudaMemcpyAsync(dst, &st, sizeof(st), cudaMemcpyHostToDevice, s);
     a.sync = fused_sync_at(base);
     // failure-path test switches, as for the CSR persistent engine
@@ -1258,9 +1258,11 @@ clsparseStatus dia_persistent_solve(DiaPcgArgs<VA, VG> a, bool learned, DiaWork&
     uint32_t grid = 0;
     cudaError_t e = cudaErrorInvalidValue;
     const int na = a.A.nd, ng = a.G.nd;
-    if (resident) {
-        e = launch_pcg_resident<VA, VG>(a, learned, plan,
-                                        word_sync_at(base, plan, a.sync.wait_ns, a.sync.never_release), s);
+    if (plan) {
+        e = test_fail("onchip-launch")
+                ? cudaErrorLaunchOutOfResources
+                : launch_pcg_resident<VA, VG>(a, learned, *plan,
+                                              word_sync_at(base, *plan, a.sync.wait_ns, a.sync.never_release), s);
     } else if (!learned) {
         if (na == 3) e = dia_launch<VA, VG, 0, 3, 3>(a, sms, s, grid);
         else if (na == 5) e = dia_launch<VA, VG, 0, 5, 3>(a, sms, s, grid);
@@ -1284,11 +1286,25 @@ clsparseStatus dia_persistent_solve(DiaPcgArgs<VA, VG> a, bool learned, DiaWork&
         cudaGetLastError();
         return clsparseInvalidKernelExecution;
     }
+    refused = false;
+    c->engine = plan ? kEngineBandedOnChip : kEngineBanded;
     if (cudaMemcpyAsync(&st, dst, sizeof(st), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return clsparseInvalidKernelExecution;
     if (st.status & kStatusBarrierTimeout) return clsparseInvalidKernelExecution;
     return clsparseSuccess;
+}
+
+template <typename VA, typename VG>
+clsparseStatus dia_persistent_solve(DiaPcgArgs<VA, VG> a, bool learned, DiaWork& w, clsparseControl c,
+                                    DiaPcgState& st) {
+    ResidentPlan plan;
+    bool refused = true;
+    clsparseStatus stt = clsparseSuccess;
+    if (resident_enabled() && resident_pcg_plan<VA, VG>(a, learned, c->sm_count, plan))
+        stt = dia_persistent_run<VA, VG>(a, learned, &plan, w, c, st, refused);
+    if (refused) stt = dia_persistent_run<VA, VG>(a, learned, nullptr, w, c, st, refused);
+    return stt;
 }
 
 }  // namespace

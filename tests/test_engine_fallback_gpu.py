@@ -109,3 +109,33 @@ def test_wait_that_runs_out_in_a_default_mode_is_not_an_error(ctrl, monkeypatch,
     run()
     assert ctrl.solver_engine() == ("banded-on-chip" if resident else "banded")
     ctrl.set_solver_loop_mode(0)
+
+
+@pytest.mark.parametrize("inner", ["fp32", "bf16"])
+def test_inner_solves_stream_when_the_chip_is_refused(ctrl, monkeypatch, inner):
+    """The refinement's inner solves: without the on-chip form's exchange area
+    or its launch they stream, with the same refinements."""
+    mat = MATS["poisson"]()
+    n = len(mat[0]) - 1
+    A = api.CsrMatrix.from_numpy(*mat)
+    A.create_meta(ctrl)
+    b = torch.tensor(np.random.default_rng(4).uniform(-1, 1, n), device="cuda")
+
+    def run():
+        x = torch.zeros(n, dtype=torch.float64, device="cuda")
+        sc = api.SolverControl(L.DIAGONAL, 5000, 1e-10, 0.0)
+        info = api.cg_mixed(x, A, b, sc, ctrl, inner=inner, inner_tol=0.1)
+        sc.release()
+        assert info["converged"] == 1
+        return info, ctrl.solver_engine()
+
+    ref, engine = run()
+    assert engine == "banded-on-chip"
+    for step in ("onchip-alloc", "onchip-launch"):
+        monkeypatch.setenv("CLSPARSE_B200_TEST_FAIL", step)
+        info, engine = run()
+        assert engine == "banded"
+        assert abs(info["outerIterations"] - ref["outerIterations"]) <= 1
+    monkeypatch.delenv("CLSPARSE_B200_TEST_FAIL")
+    monkeypatch.setenv("CLSPARSE_B200_DIA", "0")
+    assert run()[1] == "graph"
