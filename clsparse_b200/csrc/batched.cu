@@ -607,7 +607,12 @@ clsparseStatus clsparseScsrcgBatched(cldenseVector* x, const clsparseCsrMatrix* 
     // Systems of the resident kernel by CTA width and cluster size: the
     // smallest cluster that holds the system takes the least SM time (the
     // exchanges cost every CTA of a cluster alike); while the batch leaves
-    // SMs idle, all clusters are doubled.
+    // SMs idle, the clusters of systems with enough rows for it are doubled.
+    // Measured, us an iteration of one system on 128 threads, 512, and 2, 4 and 8
+    // CTAs of 512: 100 rows 2.5, 2.9, 3.5, 3.8, 4.0; 1024 rows 3.4, 3.2, 3.6,
+    // 3.7, 3.9; 1764 rows 4.1, 3.5, 3.7, 3.8, 4.0; 3600 rows -, 4.1, 4.1, 3.9,
+    // 4.0; 7056 rows -, 5.3, 4.7, 4.2, 4.2; 12,100 rows -, -, 5.5, 4.7, 4.5.
+    constexpr uint64_t kWideRows = 896, kSplitRows = 1792;
     std::vector<ResidentClass> classes(5);
     const int sizes[5][2] = {{kResWide, 8}, {kResWide, 4}, {kResWide, 2}, {kResWide, 1}, {kResSmall, 1}};
     for (int k = 0; k < 5; ++k) {
@@ -632,7 +637,10 @@ clsparseStatus clsparseScsrcgBatched(cldenseVector* x, const clsparseCsrMatrix* 
     for (int step = 0; step < 4 && ctas > 0 && 2 * ctas <= static_cast<uint64_t>(control->sm_count); ++step) {
         ctas = 0;
         for (uint32_t k = 0; k < nsys; ++k) {
-            if (at[k] > 0 && place(k, at[k] - 1)) --at[k];
+            const uint64_t rows = off[k + 1] - off[k];
+            if (at[k] > 0 && rows > (at[k] == 4 ? kWideRows : kSplitRows * static_cast<uint64_t>(sizes[at[k]][1])) &&
+                place(k, at[k] - 1))
+                --at[k];
             if (at[k] >= 0) ctas += static_cast<uint64_t>(sizes[at[k]][1]);
         }
     }

@@ -212,3 +212,32 @@ def test_batch_without_memory_leaves_x_and_a_refused_launch_is_solved_anyway(ctr
     assert float((xl - x).norm()) <= 1e-3 * float(x.norm())
     monkeypatch.delenv("CLSPARSE_B200_TEST_FAIL")
     assert torch.equal(solve()[0], x)
+
+
+def test_one_small_system_is_not_spread_over_a_cluster(ctrl):
+    """A hundred rows alone take no longer than in a batch of 148 (which has no
+    idle SMs to give them): 2.5 us an iteration, 4.0 on a cluster of eight."""
+    m = _banded_spd(100, [1, 10], seed=3)
+
+    def best(count):
+        M = sp.block_diag([m] * count, format="csr")
+        M.sort_indices()
+        A = api.CsrMatrix.from_numpy(M.indptr.astype(np.uint32), M.indices.astype(np.uint32), M.data,
+                                     dtype=torch.float32)
+        off = (np.arange(count + 1) * 100).astype(np.uint32)
+        b = torch.ones(100 * count, dtype=torch.float32, device="cuda")
+        x = torch.zeros_like(b)
+        times = []
+        for _ in range(8):
+            x.zero_()
+            sc = api.SolverControl(L.DIAGONAL, 2000, 1e-30, 0.0)
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            api.cg_batched(x, A, b, off, sc, ctrl)
+            e1.record()
+            e1.synchronize()
+            times.append(e0.elapsed_time(e1))
+            sc.release()
+        return min(times)
+
+    assert best(1) <= 1.2 * best(148)
