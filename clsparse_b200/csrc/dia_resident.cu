@@ -12,7 +12,8 @@
 // word, grid_words.cuh), and in C every CTA forms its own copy of the halo's
 // p from it, the same operations on the same values as in the owning CTA.
 // Where a CTA reaches further than its neighbours' words are worth (a halo of
-// more rows than it owns), z goes out as a plain vector ordered by the exchange.
+// more rows than it owns), z goes out as a plain vector ordered by the exchange;
+// wider still (halo_pays), the solve streams.
 //
 // What bounds it on small systems: latency, about half of it the two exchanges
 // (1.0 us each bare at 148 CTAs, see kSlotWords) and the CTA-wide sums before
@@ -1063,6 +1064,14 @@ bool plan_rows(uint32_t n, const DiaOffsets& offs, int nd_pad, int sm_count, int
     return p.rows != 0;
 }
 
+// Whether a halo is worth holding: every CTA reads all of it once an iteration,
+// which a streaming kernel's L1 and L2 do for less when it is wide beside the
+// CTA's own rows. At most `rows` rows, or twos / 2 times the CTA's own.
+bool halo_pays(const ResidentPlan& p, uint64_t rows, uint64_t twos) {
+    const uint64_t h = static_cast<uint64_t>(p.lo) + p.hi;
+    return h <= rows || 2 * h <= twos * p.mcap;
+}
+
 // Hands out the shared memory of a plan.
 struct SmemBudget {
     uint64_t left = kResidentSmem;
@@ -1103,6 +1112,12 @@ template <typename T>
 bool resident_cg_plan(uint32_t n, const DiaOffsets& offs, int nd_pad, bool jacobi, bool sym, int sm_count,
                       ResidentPlan& p) {
     if (!plan_rows(n, offs, nd_pad, sm_count, kResThreads, {2, kFewRows, kManyRows}, p)) return false;
+    // us an iteration on chip / streamed, halo rows and own rows: 8192 and 1024
+    // 7.0 / 8.1 (FP64), 6.4 / 7.8 (FP32); 12,800 and 1024 8.5 / 9.4, 7.5 / 8.3;
+    // 16,200 and 1013 9.2 / 8.8, 8.1 / 7.8; 20,000 and 3379 17.9 / 17.7, 13.1 / 15.4;
+    // 28,800 and 6811 18.4 / 19.9 (FP32); 32,768 and 3543 16.8 / 14.7; 51,200
+    // and 1384 16.8 / 9.8.
+    if (!halo_pays(p, 14336, 12)) return false;
     SmemBudget b;
     if (!b.take(static_cast<uint64_t>(p.lo) + p.mcap + p.hi, sizeof(T))) return false;
     const bool regs = p.rows <= kFewRows ? inv_in_regs<T, kFewRows>() : inv_in_regs<T, kManyRows>();
@@ -1141,6 +1156,13 @@ bool resident_pcg_plan(const DiaPcgArgs<VA, VG>& a, bool learned, int sm_count, 
     // inner iteration on 128^3 instead of 38, the diagonals still from L2 with
     // too few loads in flight beside 84 registers of vectors)
     if (!plan_rows(a.n, o, a.A.nd, sm_count, kResThreads, {kFewRows, kManyRows}, p)) return false;
+    // Jacobi, us an inner iteration on chip / streamed, halo rows and own rows:
+    // 8192 and 1024 8.0 / 8.9; 12,800 and 1024 9.3 / 9.5, and 3460 12.6 / 12.8;
+    // 16,200 and 1013 11.7 / 10.4, and 4926 14.5 / 15.5; 20,000 and 4730 15.7 /
+    // 15.0, and 6757 17.7 / 18.1. Learned (r's and q's halo beside p's): 4608 and
+    // 1024 10.1 / 11.2; 7200 and 2432 14.9 / 15.4; 8192 and 1772 14.2 / 14.2; 9800
+    // and 2318 17.8 / 16.6; 16,200 and 4926 30.2 / 23.4.
+    if (!(learned ? halo_pays(p, 7680, 2) : halo_pays(p, 12800, 7))) return false;
     SmemBudget b;
     if (!b.take(static_cast<uint64_t>(p.lo) + p.mcap + p.hi, 4)) return false;
     if (learned) {

@@ -139,3 +139,20 @@ def test_inner_solves_stream_when_the_chip_is_refused(ctrl, monkeypatch, inner):
     monkeypatch.delenv("CLSPARSE_B200_TEST_FAIL")
     monkeypatch.setenv("CLSPARSE_B200_DIA", "0")
     assert run()[1] == "graph"
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
+@pytest.mark.parametrize("reach,rows,want", [(7168, 40000, "banded-on-chip"), (7169, 40000, "banded"),
+                                             (8100, 48600, "banded"), (9000, 444000, "banded-on-chip"),
+                                             (9001, 444000, "banded")])
+def test_wide_halo_streams(ctrl, reach, rows, want, dtype):
+    """A stencil that reaches further than its halo is worth on chip streams its
+    vectors: at most 14,336 halo rows, or six times a CTA's own (444,000
+    rows on 148 SMs: 3000)."""
+    n = rows
+    v = np.full(n, 4.1)
+    A = sp.diags([np.full(n - reach, -1.0), np.full(n - 1, -1.0), v, np.full(n - 1, -1.0), np.full(n - reach, -1.0)],
+                 [-reach, -1, 0, 1, reach]).tocsr()
+    A.sort_indices()
+    mat = (A.indptr.astype(np.uint32), A.indices.astype(np.uint32), A.data)
+    assert solve(ctrl, "cg", mat, dtype=dtype)[1] == want
