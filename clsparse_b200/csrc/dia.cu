@@ -1587,6 +1587,30 @@ clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     if (meta == nullptr || meta->h_rowBlocks.size() < meta->num_words || meta->num_words < 2 ||
         meta->max_row > static_cast<uint32_t>(kMaxDiags) || (c->solver_loop_mode != 3 && !meta->few_offsets))
         return clsparseNotImplemented;
+    // Whether the streaming form beats the graph engine for nd diagonals (us an
+    // iteration, streamed / graph).
+    const auto stream_pays = [&](int nd) {
+        if (BICG) {
+            // it forms a neighbour's M p and M s from three to four vectors
+            // each: while the diagonals and the eleven work vectors stay in
+            // L2. FP64, 512^2 five-point (33 MB) 25.0 / 34.0; 1024^2 five-point (134
+            // MB) 82.6 / 81.6; 128^3 seven-point (288 MB) 191 / 161
+            return static_cast<size_t>(nd + 11) * n * sizeof(T) <= c->l2_bytes;
+        }
+        // CG: up to L2 bytes / 3.2 values of the diagonals and the seven vectors, the
+        // same for both types (39 M with 126 MB). FP64: 1100^2 five-point (14.5 M) 31 /
+        // 42, 1500^2 (27 M) 67 / 69, 140^3 seven-point (38 M) 91 / 94, 2000^2 (48 M)
+        // 117 / 118, 200^3 (112 M) 275 / 244; FP32: 1500^2 38 / 47, 140^3 56 / 61,
+        // 2000^2 83 / 74, 160^3 (57 M) 89 / 83, 200^3 172 / 159. Loop mode 3 asks for it
+        // at any size.
+        return c->solver_loop_mode == 3 || c->l2_bytes == 0 ||
+               16 * static_cast<size_t>(nd + 7) * n <= 5 * c->l2_bytes;
+    };
+    // (the least a banded matrix is padded to is three diagonals: too large for
+    // both forms without a look at its offsets)
+    if (n > static_cast<uint64_t>(std::max(1, c->sm_count)) * (BICG ? kResidentBicgRows : kResidentCgRows) &&
+        !stream_pays(3))
+        return clsparseNotImplemented;
     LaneRange lanes[kMaxLaneRanges];
     int nlanes = 0;
     for (size_t w = 0; w + 1 < meta->num_words; ++w) {
@@ -1618,18 +1642,12 @@ clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     bool has_main = false;
     for (int d = 0; d < offs.nd; ++d) has_main |= offs.off[d] == 0;
     if (ca == 0 || (jac && !has_main)) return clsparseNotImplemented;
-    // BiCGStab forms a neighbour's M p and M s from three to four vectors
-    // each: it pays while the diagonals and the eleven work vectors stay in
-    // L2. Measured per iteration on B200 against the graph engine (FP64):
-    // 512^2 five-point (33 MB) 25.0 vs 34.0 us; 1024^2 five-point (134 MB)
-    // 82.6 vs 81.6; 128^3 seven-point (288 MB) 191 vs 161. Larger systems
-    // run the graph engine.
     // On chip when the vectors fit (dia_resident.cu), else streamed through L2.
     ResidentPlan plan;
     const bool resident =
         resident_enabled() && (BICG ? resident_bicg_plan<T>(n, offs, ca, c->sm_count, plan)
                                     : resident_cg_plan<T>(n, offs, ca, jac, false, c->sm_count, plan));
-    const bool streams = !BICG || static_cast<size_t>(ca + 11) * n * sizeof(T) <= c->l2_bytes;
+    const bool streams = stream_pays(ca);
     if (!resident && !streams) return clsparseNotImplemented;
     DiaMat<T> M;
     stt = test_fail("banded-copy") ? clsparseOutOfResources : dia_build<T, T>(rp, cols, vals, n, offs, ca, w.A, s, M);

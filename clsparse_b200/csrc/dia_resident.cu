@@ -42,8 +42,8 @@ namespace {
 // of x, r and q in FP64. (1024 threads of 64 registers measured slower in FP32:
 // 6.6 us an iteration instead of 5.3 on 512^2, no change on 100^3.)
 constexpr int kResThreads = 512;
-constexpr int kFewRows = 2048 / kResThreads;    // rows per thread the kernels are built for: 4,
-constexpr int kManyRows = 7168 / kResThreads;   // 14
+constexpr int kFewRows = kResidentBicgRows / kResThreads;   // rows per thread the kernels are built for: 4,
+constexpr int kManyRows = kResidentCgRows / kResThreads;    // 14
 
 // Register arrays of R rows: D^-1 is the fourth when it fits beside x, r, q.
 template <typename T, int R>

@@ -50,6 +50,9 @@ struct ResidentPlan {
     size_t smem = 0;
 };
 
+// Rows a CTA of the drop-in CG / BiCGStab holds at most.
+constexpr uint32_t kResidentCgRows = 7168, kResidentBicgRows = 2048;
+
 // Whether a solve runs on chip, and its layout: the drop-in CG and BiCGStab on
 // n rows, the refinement's inner PCG. `sym`: A is symmetric bit for bit, its
 // offsets symmetric, no padding diagonals.

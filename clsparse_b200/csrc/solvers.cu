@@ -841,11 +841,14 @@ clsparseStatus cg_solve(cldenseVector* xv, const clsparseCsrMatrix* A, const cld
     // cooperative launch over a diagonal-storage copy (dia.cu); other matrices,
     // and the options that engine does not carry (history, snapshots, extended
     // precision, the refinement's continued solves), stay on the engines below.
-    // Modes 0 and 1 (which give the same iterates) take it because it is faster wherever it applies, per iteration
-    // (FP64, graph engine / banded): 512^2 five-point 17.3 / 6.0 us, 1000^2
-    // 34.0 / 16.5, 64^3 seven-point 18.5 / 8.5, 100^3 45.4 / 29.2, 128^3
-    // (streamed) 75 / 71, and a solve of 3,600 rows 3.0 / 1.05 ms. Matrices with
-    // more column offsets than it keeps are known from their meta.
+    // Modes 0 and 1 (which give the same iterates) take it where it is faster (the
+    // rules are in dia.cu and dia_resident.cu). Per iteration on chip / graph engine
+    // (FP64): 512^2 five-point 6.0 / 17.3 us, 1000^2 16.5 / 34.0, 64^3 seven-point 8.5 /
+    // 18.5, 100^3 29.2 / 45.4. The copy is laid out at every call, and a whole
+    // solve of one and of five iterations takes, against the graph engine with its
+    // graph at hand, 16^2: 105 / 92 and 120 / 135 us; 512^2: 116 / 126 and 143 / 197;
+    // 128^3 (streamed): 387 / 599 and 676 / 887; on new buffers, which cost the
+    // graph engine a capture, one iteration on 512^2: 111 / 413.
     if (c->solver_loop_mode != 2 && std::is_same_v<V, T> && ws == nullptr && n > 0 && !c->extended_precision &&
         sc->history == nullptr && sc->snapshotCount == 0 && dia_enabled()) {
         stt = dia_cg_dropin<T>(xv, A, bv, sc, c);

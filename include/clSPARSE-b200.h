@@ -247,9 +247,10 @@ cldenseDdotNoAlloc(clsparseScalar* r, const cldenseVector* x, const cldenseVecto
  * the device at once and device memory for the copy: where either is refused
  * the solve runs as below, as it does in modes 0 and 1 when a wait of the
  * kernel's CTAs for one another runs out (4 s); mode 3 then returns
- * clsparseInvalidKernelExecution. Other matrices (no meta, not
- * banded), a zero or missing diagonal under Jacobi, residual history or
- * snapshots, extended precision, and BiCGStab systems larger than L2 run as
+ * clsparseInvalidKernelExecution. Other matrices (no meta, not banded), a zero
+ * or missing diagonal under Jacobi, residual history or snapshots, extended
+ * precision, BiCGStab systems larger than L2 and, in modes 0 and 1, CG systems
+ * of more than L2 bytes / 3.2 values of the diagonals and seven vectors run as
  * 0 = one CUDA graph per solve with a device-side conditional WHILE node (no
  * host round trip per iteration; the default); 1 = host-enqueued chunks of
  * iterations with a device done flag (same iterates as 0); 2 = CG and

@@ -156,3 +156,20 @@ def test_wide_halo_streams(ctrl, reach, rows, want, dtype):
     A.sort_indices()
     mat = (A.indptr.astype(np.uint32), A.indices.astype(np.uint32), A.data)
     assert solve(ctrl, "cg", mat, dtype=dtype)[1] == want
+
+
+@pytest.mark.parametrize("kind,dtype", [("cg", torch.float64), ("cg", torch.float32), ("bicgstab", torch.float64)],
+                         ids=["cg-f64", "cg-f32", "bicgstab-f64"])
+def test_large_solves_run_on_the_faster_engine(ctrl, kind, dtype):
+    """The default modes leave a CG whose diagonals and vectors are more than
+    L2 bytes / 3.2 values, and a BiCGStab whose are more than L2, to the graph
+    engine, which is faster there; loop mode 3 streams the CG at any size. A
+    tridiagonal matrix on both sides of the line."""
+    l2 = torch.cuda.get_device_properties(0).L2_cache_size
+    n = l2 * 5 // 160 if kind == "cg" else l2 // (14 * 8)
+    for rows, want in ((n, "banded"), (n + 1, "graph")):
+        A = sp.diags([np.full(rows - 1, -1.0), np.full(rows, 4.1), np.full(rows - 1, -1.0)], [-1, 0, 1]).tocsr()
+        mat = (A.indptr.astype(np.uint32), A.indices.astype(np.uint32), A.data)
+        assert solve(ctrl, kind, mat, dtype=dtype)[1] == want
+        if kind == "cg":
+            assert solve(ctrl, kind, mat, mode=3, dtype=dtype)[1] == "banded"
