@@ -146,3 +146,70 @@ def test_csrmm_vector_widths(ctrl, dtype, ncols, pad, off):
     out = raw[off:].reshape(n, ld)
     assert np.max(np.abs(out[:, :ncols] - ref) / scale) <= TOL[dtype] * 10
     np.testing.assert_array_equal(out[:, ncols:], 0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
+@pytest.mark.parametrize("major", ["row", "col"])
+@pytest.mark.parametrize("ncols", [1, 2, 3, 4, 8, 16, 31, 32, 33, 65, 100])
+def test_csrmm_short_rows(ctrl, dtype, ncols, major):
+    """The form for rows of fewer than 8 nonzeros on average: every remainder of
+    its 4, 2 and 1 steps, long rows among short ones, full and narrow tiles, and
+    the other form for the same matrix when a meta shows a long row. Tolerance
+    as above (at most 1500 products: the absolute sum scales)."""
+    mj = L.rowMajor if major == "row" else L.columnMajor
+    lens = [0, 1, 2, 3, 4, 5, 6, 7, 9, 11, 15, 17, 31, 33, 0, 0] * 6 + [1] * 400 + [1500]
+    n, m = len(lens), 1600
+    rp, col, val = matgen.random_lengths(lens, m, seed=ncols)
+    assert len(val) < 8 * n
+    rng = np.random.default_rng(ncols)
+    B, C0 = rng.uniform(-1, 1, (m, ncols)), rng.uniform(-1, 1, (n, ncols))
+    ldb, ldc = (ncols, ncols) if mj == L.rowMajor else (m, n)
+    t = np.float64 if dtype == torch.float64 else np.float32
+    Am = sp.csr_matrix((np.asarray(val, t).astype(np.float64), col.astype(np.int64), rp.astype(np.int64)), shape=(n, m))
+    Bc, Cc = np.asarray(B, t).astype(np.float64), np.asarray(C0, t).astype(np.float64)
+    ref = -0.75 * (Am @ Bc) + 0.5 * Cc
+    scale = 0.75 * (abs(Am) @ abs(Bc)) + 0.5 * abs(Cc) + 1e-300
+    a = torch.tensor([-0.75], dtype=dtype, device="cuda")
+    b = torch.tensor([0.5], dtype=dtype, device="cuda")
+    fn = api.lib().clsparseDcsrmm if dtype == torch.float64 else api.lib().clsparseScsrmm
+    for meta in (False, True):
+        A = api.CsrMatrix.from_numpy(rp, col, val, num_cols=m, dtype=dtype)
+        if meta:
+            A.create_meta(ctrl)
+        tb, tc = layout(B, ldb, mj, dtype), layout(C0, ldc, mj, dtype)
+        db, dc = dense(tb, m, ncols, ldb, mj), dense(tc, n, ncols, ldc, mj)
+        assert fn(C.byref(api.scalar(a)), C.byref(A.s), C.byref(db), C.byref(api.scalar(b)), C.byref(dc), ctrl.handle) == 0
+        out = unlayout(tc, n, ncols, ldc, mj)
+        assert np.max(np.abs(out - ref) / scale) <= TOL[dtype] * 10
+
+
+def test_csrmm_short_rows_are_not_slower_than_columns_one_by_one(ctrl):
+    """One column of a five-point matrix takes no longer than two products
+    of the same matrix with a vector (as long as five before short rows had a
+    form of their own)."""
+    rp, col, val = matgen.poisson2d(600)
+    n = len(rp) - 1
+    A = api.CsrMatrix.from_numpy(rp, col, val)
+    A.create_meta(ctrl)
+    B, Cm = (torch.rand(n, dtype=torch.float64, device="cuda") for _ in range(2))
+    one, zero = torch.ones(1, dtype=torch.float64, device="cuda"), torch.zeros(1, dtype=torch.float64, device="cuda")
+    db, dc = dense(B, n, 1, 1, L.rowMajor), dense(Cm, n, 1, 1, L.rowMajor)
+
+    def best(fn):
+        times = []
+        for _ in range(10):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(10):
+                fn()
+            e1.record()
+            e1.synchronize()
+            times.append(e0.elapsed_time(e1))
+        return min(times)
+
+    ctrl.enable_async(True)
+    mm = best(lambda: api.lib().clsparseDcsrmm(C.byref(api.scalar(one)), C.byref(A.s), C.byref(db),
+                                               C.byref(api.scalar(zero)), C.byref(dc), ctrl.handle))
+    mv = best(lambda: api.csrmv(one, A, B, zero, Cm, ctrl))
+    ctrl.enable_async(False)
+    assert mm <= 2 * mv, (mm, mv)
