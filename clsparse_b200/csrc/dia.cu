@@ -60,6 +60,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <limits>
+#include <new>
 #include <type_traits>
 #include <vector>
 
@@ -113,8 +114,8 @@ __device__ bool set_insert(int32_t* table, int32_t o) {
 }
 
 // The distinct offsets cols[k] - i of a CSR matrix into `table` (kSlots
-// entries preset to kEmpty); flags[0] |= 1 when there are more than the set
-// holds, |= 2 when a row's columns are not strictly increasing.
+// entries preset to kEmpty); bits of flags[0]: 1 when there are more than the set
+// holds, 2 when a row's columns are not strictly increasing.
 __global__ void dia_offsets_kernel(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ cols, uint32_t n,
                                    int32_t* table, int* flags) {
     __shared__ int32_t st[kSlots];
@@ -1078,6 +1079,28 @@ bool dia_enabled() {
     return !(e && e[0] == '0' && e[1] == '\0');
 }
 
+cudaError_t launch_band_probe(const uint32_t* rp, const uint32_t* cols, uint32_t n, int32_t* words, cudaStream_t s) {
+    static_assert(kBandProbeWords == kSlots + 1 && kBandDiags == kMaxDiags, "the table and its flags");
+    const cudaError_t e = cudaMemsetAsync(words, 0x80, kBandProbeWords * sizeof(int32_t), s);  // kEmpty in every slot
+    if (e != cudaSuccess) return e;
+    dia_offsets_kernel<<<std::min<uint32_t>((n + 255) / 256, 1184), 256, 0, s>>>(rp, cols, n, words, words + kSlots);
+    return cudaGetLastError();
+}
+
+int band_probe_result(const int32_t* words, uint32_t n, uint32_t nnz, int32_t (&offsets)[kBandDiags]) {
+    if (words[kSlots] != kEmpty) return 0;  // (the flags start as an empty slot)
+    int nd = 0;
+    for (int k = 0; k < kSlots; ++k) {
+        if (words[k] == kEmpty) continue;
+        if (nd == kBandDiags) return 0;
+        offsets[nd++] = words[k];
+    }
+    // at least half of the stored diagonal entries hold matrix entries
+    if (static_cast<uint64_t>(nnz) * 2 < static_cast<uint64_t>(nd) * n) return 0;
+    std::sort(offsets, offsets + nd);
+    return nd;
+}
+
 clsparseStatus dia_detect(const uint32_t* rp, const uint32_t* cols, uint32_t n, uint32_t nnz, DiaWork& w,
                           cudaStream_t s, DiaOffsets& offs) {
     offs.nd = 0;
@@ -1087,46 +1110,13 @@ clsparseStatus dia_detect(const uint32_t* rp, const uint32_t* cols, uint32_t n, 
         return clsparseOutOfResources;
     }
     int32_t* table = static_cast<int32_t*>(w.table.ptr);
-    int* flags = reinterpret_cast<int*>(table + kSlots);
-    cudaMemsetAsync(table, 0x80, kSlots * sizeof(int32_t), s);  // kEmpty in every slot
-    cudaMemsetAsync(flags, 0, sizeof(int), s);
-    const uint32_t grid = std::min<uint32_t>((n + 255) / 256, 1184);
-    dia_offsets_kernel<<<grid, 256, 0, s>>>(rp, cols, n, table, flags);
-    int32_t h[kSlots + 1];
-    if (cudaGetLastError() != cudaSuccess ||
+    int32_t h[kBandProbeWords];
+    if (launch_band_probe(rp, cols, n, table, s) != cudaSuccess ||
         cudaMemcpyAsync(h, table, sizeof(h), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return clsparseInvalidKernelExecution;
-    if (h[kSlots] != 0) return clsparseInvalidValue;
-    std::vector<int32_t> o;
-    for (int k = 0; k < kSlots; ++k)
-        if (h[k] != kEmpty) o.push_back(h[k]);
-    if (o.empty() || o.size() > static_cast<size_t>(kMaxDiags)) return clsparseInvalidValue;
-    // at least half of the stored diagonal entries hold matrix entries
-    if (static_cast<uint64_t>(nnz) * 2 < static_cast<uint64_t>(o.size()) * n) return clsparseInvalidValue;
-    std::sort(o.begin(), o.end());
-    offs.nd = static_cast<int>(o.size());
-    for (int d = 0; d < offs.nd; ++d) offs.off[d] = o[d];
-    return clsparseSuccess;
-}
-
-bool dia_few_offsets(const uint32_t* rp, const uint32_t* cols, uint32_t n, uint32_t max_row, cudaStream_t s) {
-    if (n == 0 || max_row == 0 || max_row > static_cast<uint32_t>(kMaxDiags)) return false;
-    DeviceBuffer table;
-    if (table.ensure(kSlots * sizeof(int32_t) + 64) != cudaSuccess) {
-        cudaGetLastError();
-        return true;  // (not known: the solve looks)
-    }
-    int32_t* t = static_cast<int32_t*>(table.ptr);
-    int* flags = reinterpret_cast<int*>(t + kSlots);
-    cudaMemsetAsync(t, 0x80, kSlots * sizeof(int32_t), s);
-    cudaMemsetAsync(flags, 0, sizeof(int), s);
-    dia_offsets_kernel<<<std::min<uint32_t>((n + 255) / 256, 1184), 256, 0, s>>>(rp, cols, n, t, flags);
-    int h = 0;
-    if (cudaGetLastError() != cudaSuccess || cudaMemcpyAsync(&h, flags, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
-        return true;
-    return (h & 1) == 0;
+    offs.nd = band_probe_result(h, n, nnz, offs.off);
+    return offs.nd > 0 ? clsparseSuccess : clsparseInvalidValue;
 }
 
 template <typename VI, typename VO>
@@ -1490,7 +1480,8 @@ clsparseStatus dropin_run(cldenseVector* xv, const clsparseCsrMatrix* A, const c
         }
     }
 
-    DiaCgState h;
+    static_assert(sizeof(DiaCgState) <= 512 && std::is_trivially_copyable_v<DiaCgState>);
+    DiaCgState& h = *new (static_cast<char*>(c->pinned) + 1024) DiaCgState();  // (1024 .. 1535: free between solves)
     h.rel_tol = sc->relativeTolerance;
     h.abs_tol = sc->absoluteTolerance;
     h.max_iters = sc->maxIters;
@@ -1585,7 +1576,7 @@ clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     // kMaxLaneRanges, leaves the solve to the graph engine.
     const auto* meta = static_cast<const matrix_meta*>(A->meta);
     if (meta == nullptr || meta->h_rowBlocks.size() < meta->num_words || meta->num_words < 2 ||
-        meta->max_row > static_cast<uint32_t>(kMaxDiags) || (c->solver_loop_mode != 3 && !meta->few_offsets))
+        meta->max_row > static_cast<uint32_t>(kMaxDiags) || (c->solver_loop_mode != 3 && meta->band_diags == 0))
         return clsparseNotImplemented;
     // Whether the streaming form beats the graph engine for nd diagonals (us an
     // iteration, streamed / graph).
@@ -1606,10 +1597,12 @@ clsparseStatus dia_dropin(cldenseVector* xv, const clsparseCsrMatrix* A, const c
         return c->solver_loop_mode == 3 || c->l2_bytes == 0 ||
                16 * static_cast<size_t>(nd + 7) * n <= 5 * c->l2_bytes;
     };
-    // (the least a banded matrix is padded to is three diagonals: too large for
-    // both forms without a look at its offsets)
+    // (too large for both forms with the offsets it had when its meta was made:
+    // no look at its offsets)
+    int made = 3, unused = 0;
+    if (meta->band_diags > 0) dia_classes(meta->band_diags, 0, false, made, unused);
     if (n > static_cast<uint64_t>(std::max(1, c->sm_count)) * (BICG ? kResidentBicgRows : kResidentCgRows) &&
-        !stream_pays(3))
+        !stream_pays(made))
         return clsparseNotImplemented;
     LaneRange lanes[kMaxLaneRanges];
     int nlanes = 0;

@@ -132,7 +132,7 @@ struct matrix_meta {
     uint32_t nnz_lo = 0;                // row_pointer[0]
     uint32_t nnz_hi = 0;                // row_pointer[num_rows]
     uint32_t max_row = 0;               // longest row (nonzeros)
-    bool few_offsets = false;           // at most 64 distinct column offsets when it was made: solves look closer
+    int band_diags = 0;                 // distinct column offsets when it was made (0: not banded): solves look closer
     int device = 0;
     int sm_count = 148;                 // SMs of the device the meta was made on
     // Row-block shape the words were made with (the reference's constants by
@@ -257,10 +257,15 @@ struct CsrView {
 cudaError_t launch_validate_columns(const uint32_t* cols, size_t n, uint32_t ncols, int* bad, int sm_count,
                                     cudaStream_t s);
 
-// Whether a CSR matrix may be banded: false when its columns have more distinct
-// offsets from their rows than the banded engine's detection keeps (dia.cu).
-// clsparseCsrMetaCreate asks once, so that solves of other matrices need not.
-bool dia_few_offsets(const uint32_t* rp, const uint32_t* cols, uint32_t n, uint32_t max_row, cudaStream_t s);
+// Looks for a banded matrix (dia.cu): launches the search over the columns'
+// offsets from their rows into kBandProbeWords words of device memory; their
+// host copy gives the sorted offsets (at most kBandDiags; 0: not banded -- more of
+// them, unsorted rows, or mostly empty diagonals). clsparseCsrMetaCreate asks
+// once, so that solves of other matrices need not.
+constexpr int kBandDiags = 16;
+constexpr int kBandProbeWords = 65;
+cudaError_t launch_band_probe(const uint32_t* rp, const uint32_t* cols, uint32_t n, int32_t* words, cudaStream_t s);
+int band_probe_result(const int32_t* words, uint32_t n, uint32_t nnz, int32_t (&offsets)[kBandDiags]);
 
 // Number of CTAs an SpMV of this matrix launches (sizes epilogue partials).
 uint32_t spmv_num_ctas(const matrix_meta* meta, uint32_t nrows, uint32_t nnz);

@@ -228,6 +228,9 @@ int default_cta_threads() {
     return nt;
 }
 
+// Device words behind the meta's error flag: the search for a banded matrix.
+constexpr int kProbeAt = 16;
+
 clsparseStatus create_meta(clsparseCsrMatrix* csrMatx, clsparseControl control, uint32_t blk, uint32_t mult,
                            uint32_t rfv, int nt) {
     clsparseStatus st = check_entry(control);
@@ -281,7 +284,7 @@ clsparseStatus create_meta(clsparseCsrMatrix* csrMatx, clsparseControl control, 
         cudaMalloc(&meta->d_word_nnz, w * sizeof(uint32_t)) != cudaSuccess ||
         cudaMalloc(&meta->d_lr_partial, w * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&meta->d_lr_ticket, w * sizeof(uint32_t)) != cudaSuccess ||
-        cudaMalloc(&meta->d_error, sizeof(int)) != cudaSuccess) {
+        cudaMalloc(&meta->d_error, (kProbeAt + kBandProbeWords) * sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
         return clsparseOutOfResources;
     }
@@ -299,17 +302,28 @@ clsparseStatus create_meta(clsparseCsrMatrix* csrMatx, clsparseControl control, 
         e = launch_validate_columns(dev_ptr<const uint32_t>(csrMatx->col_indices, csrMatx->off_col_indices) + rp.front(),
                                     csrMatx->num_nonzeros, static_cast<uint32_t>(csrMatx->num_cols), meta->d_error,
                                     meta->sm_count, control->stream);
-    int bad = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, meta->d_error, sizeof(int), cudaMemcpyDeviceToHost, control->stream);
+    // and, in the same wait, whether the matrix is banded
+    const uint32_t n = static_cast<uint32_t>(csrMatx->num_rows);
+    const bool probe = n > 0 && meta->max_row > 0 && meta->max_row <= static_cast<uint32_t>(kBandDiags);
+    if (e == cudaSuccess && probe)
+        e = launch_band_probe(dev_ptr<const uint32_t>(csrMatx->row_pointer, csrMatx->off_row_pointer),
+                              dev_ptr<const uint32_t>(csrMatx->col_indices, csrMatx->off_col_indices), n,
+                              meta->d_error + kProbeAt, control->stream);
+    int32_t found[kProbeAt + kBandProbeWords] = {};
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(found, meta->d_error, probe ? sizeof(found) : sizeof(int), cudaMemcpyDeviceToHost,
+                            control->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(control->stream);
     if (e != cudaSuccess) return clsparseInvalidKernelExecution;
-    if (bad) return clsparseInvalidValue;
+    if (found[0]) return clsparseInvalidValue;
+    if (probe) {
+        int32_t offsets[kBandDiags];
+        meta->band_diags =
+            band_probe_result(found + kProbeAt, n, static_cast<uint32_t>(csrMatx->num_nonzeros), offsets);
+    }
     if (cudaMemsetAsync(meta->d_error, 0, sizeof(int), control->stream) != cudaSuccess ||
         cudaStreamSynchronize(control->stream) != cudaSuccess)
         return clsparseInvalidKernelExecution;
-    meta->few_offsets = dia_few_offsets(dev_ptr<const uint32_t>(csrMatx->row_pointer, csrMatx->off_row_pointer),
-                                        dev_ptr<const uint32_t>(csrMatx->col_indices, csrMatx->off_col_indices),
-                                        static_cast<uint32_t>(csrMatx->num_rows), meta->max_row, control->stream);
     meta->h_word_nnz = std::move(word_nnz);
     csrMatx->meta = meta.release();
     return clsparseSuccess;

@@ -5,6 +5,8 @@ The failures are made on the host (CLSPARSE_B200_TEST_FAIL names the step that
 reports failure without being tried)."""
 from __future__ import annotations
 
+import time
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -173,3 +175,39 @@ def test_large_solves_run_on_the_faster_engine(ctrl, kind, dtype):
         assert solve(ctrl, kind, mat, dtype=dtype)[1] == want
         if kind == "cg":
             assert solve(ctrl, kind, mat, mode=3, dtype=dtype)[1] == "banded"
+
+
+def test_solves_of_matrices_that_are_not_banded_pay_nothing(ctrl, monkeypatch):
+    """A matrix of short rows with more column offsets than the banded engine
+    takes is known from its meta: a solve of one iteration takes no longer than with
+    that engine off (with a search at every solve: 140 us instead of 100)."""
+    rng = np.random.default_rng(3)
+    n = 20000
+    S = sp.csr_matrix((n, n))
+    for o in np.unique(rng.integers(1, n // 3, 15)):
+        S = S + sp.diags([-rng.uniform(0.1, 1, n - o) * (rng.uniform(size=n - o) < 0.2)], [o], shape=(n, n))
+    S = S + S.T
+    S = (S + sp.diags([np.asarray(abs(S).sum(axis=1)).ravel() + 0.3], [0])).tocsr()
+    S.eliminate_zeros()
+    S.sort_indices()
+    assert np.diff(S.indptr).max() <= 16
+    A = api.CsrMatrix.from_numpy(S.indptr.astype(np.uint32), S.indices.astype(np.uint32), S.data)
+    A.create_meta(ctrl)
+    b = torch.ones(n, dtype=torch.float64, device="cuda")
+    x = torch.zeros_like(b)
+
+    def best():
+        times = []
+        for _ in range(40):
+            sc = api.SolverControl(L.DIAGONAL, 1, 0.0, 0.0)
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            api.solve("cg", x, A, b, sc, ctrl)
+            times.append(time.perf_counter() - t)
+            sc.release()
+        return min(times)
+
+    default = best()
+    assert ctrl.solver_engine() == "graph"
+    monkeypatch.setenv("CLSPARSE_B200_DIA", "0")
+    assert default <= 1.15 * best()
