@@ -969,11 +969,15 @@ clsparseStatus bicg_solve(cldenseVector* xv, const clsparseCsrMatrix* A, const c
     DeviceGuard guard(c->device);
     const size_t n = A->num_rows;
     // loop modes 0, 1 and 3 on a banded matrix: one cooperative launch (see
-    // cg_solve). BiCGStab's iteration count moves by a few with the order of the
-    // dot products' sums, and on the reference's own small runs (up to 400 rows)
-    // the graph engine's order keeps it within the pinned two: modes 0 and 1 take
-    // the banded engine from kBandedBicgRows on (90,000 rows: 31.7 -> 8.8 us an
-    // iteration).
+    // cg_solve); modes 0 and 1 from kBandedBicgRows on. BiCGStab's iteration count
+    // depends on the order of the dot products' sums. The reference's own runs (up to
+    // 512 rows) are met within max(2, 5 %) by the graph engine's order, not by the
+    // banded one's (47 against 44 on one), so systems of such sizes stay there,
+    // although its iteration takes 26 us and the banded one's 7.4 (1024 to 2304
+    // rows alike). On longer runs neither order is that close: 234 runs of 13
+    // matrices of 2304 to 22,500 rows (both types, both preconditioners, 1e-4 to
+    // 1e-10) against the oracle, 58 of the graph engine's counts are outside that bar and 39 of
+    // the banded engine's, by 3.6 % and 2.7 % on average.
     constexpr size_t kBandedBicgRows = 2048;
     if ((c->solver_loop_mode == 3 || (c->solver_loop_mode != 2 && n >= kBandedBicgRows)) && std::is_same_v<V, T> && n > 0 && !c->extended_precision &&
         sc->history == nullptr && dia_enabled()) {

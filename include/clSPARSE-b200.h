@@ -243,7 +243,9 @@ cldenseDdotNoAlloc(clsparseScalar* r, const cldenseVector* x, const cldenseVecto
  * rebuilt at every call (the reference's row order and rounding, stop tests,
  * nIters and solver-control bookkeeping; iterates equal up to the order of
  * the dot-product sums), with the vectors held on chip where they fit;
- * BiCGStab in modes 0 and 1 from 2048 rows on. That kernel needs every SM of
+ * BiCGStab in modes 0 and 1 from 2048 rows on (its iteration count depends on
+ * the order of the dot products' sums: on either engine a few per cent from the
+ * reference's on long runs). That kernel needs every SM of
  * the device at once and device memory for the copy: where either is refused
  * the solve runs as below, as it does in modes 0 and 1 when a wait of the
  * kernel's CTAs for one another runs out (4 s); mode 3 then returns
