@@ -241,3 +241,31 @@ def test_threads_with_different_plans(ctrl):
     for t in threads:
         t.join()
     assert not errors, errors[0]
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
+@pytest.mark.parametrize("case", [(1000000, [1, 1000]), (1060864, [1, 1030]), (700001, [1, 60, 3000]), (20000, [1, 150])],
+                         ids=_case_id)
+def test_lower_diagonals_from_the_upper_ones(ctrl, monkeypatch, case, dtype):
+    """CLSPARSE_B200_DIA_SYM on chip: never (0), wherever possible (1) and the
+    default (where not every diagonal fits) give the same x bit for bit."""
+    n, offs = case
+    rp, col, val = banded(n, offs, seed=n)
+    A = api.CsrMatrix.from_numpy(rp, col, val, dtype=dtype)
+    A.create_meta(ctrl)
+    b = torch.tensor(np.random.default_rng(7).uniform(-1, 1, n), dtype=dtype, device="cuda")
+
+    def solve(mode):
+        if mode is None:
+            monkeypatch.delenv("CLSPARSE_B200_DIA_SYM", raising=False)
+        else:
+            monkeypatch.setenv("CLSPARSE_B200_DIA_SYM", mode)
+        x = torch.zeros_like(b)
+        sc = api.SolverControl(L.DIAGONAL, 25, 0.0, 0.0)
+        api.solve("cg", x, A, b, sc, ctrl)
+        sc.release()
+        assert ctrl.solver_engine() == "banded-on-chip"
+        return x
+
+    x0, x1, xd = solve("0"), solve("1"), solve(None)
+    assert torch.equal(x0, x1) and torch.equal(x0, xd)
