@@ -117,7 +117,7 @@ __device__ __forceinline__ uint32_t first_at_least(const uint32_t* __restrict__ 
 // above its predecessor's, has the pointers in between to write; the last
 // position's also those behind its row. More than kShortGap of them are written
 // by its warp, a lane each. Whole chunks [c kGapRows, (c + 1) kGapRows) without a step,
-// as long runs of empty rows hold, are left to the CTAs behind the runs, a
+// as long runs of empty rows hold, are left to the CTAs before the runs, a
 // thread per chunk to look it up and a warp to write it: the pointers are
 // spread over the device however the nonzeros lie. Both ends of the rule
 // measured, coo2csr with its wait: 10 M rows with 3000 nonzeros 644 us with every
@@ -151,15 +151,15 @@ __device__ __forceinline__ void fill_gap_chunks(const uint32_t* __restrict__ ri,
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
     coo_to_csr_kernel(const uint32_t* __restrict__ ri, const uint32_t* __restrict__ ci, const T* __restrict__ vi,
-                      uint32_t nnz, uint32_t nrows, uint32_t runs, uint32_t* __restrict__ rp,
+                      uint32_t nnz, uint32_t nrows, uint32_t gap_ctas, uint32_t* __restrict__ rp,
                       uint32_t* __restrict__ co, T* __restrict__ vo) {
     constexpr uint32_t PER = kChunk / kThreads;
-    if (blockIdx.x >= runs) {
-        fill_gap_chunks(ri, nnz, nrows, blockIdx.x - runs, rp);
+    if (blockIdx.x < gap_ctas) {  // (first: their look-ups are chains of loads)
+        fill_gap_chunks(ri, nnz, nrows, blockIdx.x, rp);
         return;
     }
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t b = blockIdx.x * kChunk;
+    const uint32_t b = (blockIdx.x - gap_ctas) * kChunk;
     const uint32_t e = static_cast<uint32_t>(min(static_cast<uint64_t>(nnz), static_cast<uint64_t>(b) + kChunk));
     uint32_t row[PER], prev[PER];
 #pragma unroll
@@ -171,11 +171,23 @@ __global__ void __launch_bounds__(kThreads)
     Run<T> run;
     run.load(ci, vi, co, vo, b, e);
     run.store(ci, vi, co, vo, b, e);
-    // rp[from, to) = at but for the whole chunks inside; by every lane of the warp
-    auto fill = [&](uint32_t from, uint32_t to, uint32_t at) {
-        const bool any = from < to, lng = any && to - from > kShortGap;
-        if (any && !lng)
-            for (uint32_t r = from; r < to; ++r) rp[r] = at;
+    // the pointers [from, to) of position k, and the last one's [row + 1, nrows)
+    auto from_of = [&](uint32_t u, uint32_t k) { return k > 0 ? (prev[u] < nrows ? prev[u] + 1 : nrows) : 0; };
+    auto to_of = [&](uint32_t u) { return row[u] < nrows ? row[u] + 1 : nrows; };
+    bool any_long = e == nnz;
+#pragma unroll
+    for (uint32_t u = 0; u < PER; ++u) {
+        const uint32_t k = b + u * kThreads + threadIdx.x;
+        if (k >= e) continue;
+        const uint32_t from = from_of(u, k), to = to_of(u);
+        if (to > from && to - from > kShortGap)
+            any_long = true;
+        else
+            for (uint32_t r = from; r < to; ++r) rp[r] = k;
+    }
+    if (!__any_sync(0xffffffffu, any_long)) return;
+    // long ones, by every lane of the warp, but for the whole chunks inside
+    auto fill = [&](bool lng, uint32_t from, uint32_t to, uint32_t at) {
         for (unsigned todo = __ballot_sync(0xffffffffu, lng); todo;) {
             // four gaps at a time (the last one again where fewer are left)
             int l = 0;
@@ -198,25 +210,14 @@ __global__ void __launch_bounds__(kThreads)
     for (uint32_t u = 0; u < PER; ++u) {
         const uint32_t k = b + u * kThreads + threadIdx.x;
         const bool on = k < e;
-        fill(on && k > 0 ? (prev[u] < nrows ? prev[u] + 1 : nrows) : 0, on ? (row[u] < nrows ? row[u] + 1 : nrows) : 0, k);
+        const uint32_t from = from_of(u, k), to = to_of(u);
+        fill(on && to > from && to - from > kShortGap, from, to, k);
         if (e == nnz) {
             const bool last = on && k == nnz - 1;
-            fill(last && row[u] < nrows ? row[u] + 1 : nrows, nrows, nnz);
+            fill(last && to < nrows, to, nrows, nnz);
             if (last) rp[nrows] = nnz;
         }
     }
-}
-
-// The row of position k: the last with rp[row] <= k.
-__device__ __forceinline__ uint32_t row_of(const uint32_t* __restrict__ rp, uint32_t lo, uint32_t hi, uint32_t k) {
-    while (hi - lo > 1) {
-        const uint32_t mid = lo + (hi - lo) / 2;
-        if (__ldg(rp + mid) <= k)
-            lo = mid;
-        else
-            hi = mid;
-    }
-    return lo;
 }
 
 // Row index of every position of a run: the rows that start inside it mark
@@ -227,33 +228,53 @@ __device__ __forceinline__ uint32_t row_of(const uint32_t* __restrict__ rp, uint
 // pointers a thread). 10 M rows with 3000 nonzeros: 6.1 ms walking, 44 us here.
 constexpr uint32_t kWalkRows = 4 * kChunk;
 template <typename T>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 8)  // (32 registers: the looking up, rare, may spill)
     csr_to_coo_kernel(const uint32_t* __restrict__ rp, const uint32_t* __restrict__ ci, const T* __restrict__ vi,
                       uint32_t nnz, uint32_t nrows, uint32_t* __restrict__ ro, uint32_t* __restrict__ co,
                       T* __restrict__ vo) {
     constexpr uint32_t PER = kChunk / kThreads;  // consecutive positions of a thread in the scan
     __shared__ uint32_t mark[kChunk];
     __shared__ uint32_t warp_max[kThreads / 32];
-    __shared__ uint32_t bounds[2];
+    __shared__ uint32_t first;
     const uint32_t b = blockIdx.x * kChunk;
     const uint32_t e = static_cast<uint32_t>(min(static_cast<uint64_t>(nnz), static_cast<uint64_t>(b) + kChunk));
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint32_t rows_b = __ldg(rp), rows_e = __ldg(rp + nrows);  // positions outside the rows stay as they are
     Run<T> run;
     run.load(ci, vi, co, vo, b, e);
-    if (t < 2) bounds[t] = row_of(rp, 0, nrows, t == 0 ? b : e - 1);
+    if (t == 0) {
+        // the row of position b: the last with rp[row] <= b
+        uint32_t lo = 0, hi = nrows;
+        while (hi - lo > 1) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if (__ldg(rp + mid) <= b)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        first = lo;
+    }
     for (uint32_t i = t; i < kChunk; i += kThreads) mark[i] = 0;
     run.store(ci, vi, co, vo, b, e);
     __syncthreads();
-    const uint32_t r0 = bounds[0], r1 = max(r0, bounds[1]);  // the rows of the first and the last position
-    if (r1 - r0 > kWalkRows) {
+    const uint32_t r0 = first;
+    // rows after the first that start inside the run (empty ones share a
+    // position with the next: the largest stays)
+    const bool far = nrows - r0 > kWalkRows && __ldg(rp + r0 + kWalkRows) < e;  // (the same in every thread)
+    if (!far) {
+        for (uint32_t r = r0 + 1 + t; r < nrows; r += kThreads) {
+            const uint32_t at = __ldg(rp + r);
+            if (at >= e) break;
+            if (at >= b) atomicMax(&mark[at - b], r);
+        }
+    } else {
         uint32_t lo[PER], hi[PER];
 #pragma unroll
         for (uint32_t u = 0; u < PER; ++u) {
             lo[u] = r0;
-            hi[u] = r1 + 1;
+            hi[u] = nrows;
         }
-        for (uint32_t w = r1 - r0; w > 0; w >>= 1)  // (halvings of r1 - r0 + 1 rows)
+        for (uint32_t w = nrows - r0; w > 0; w >>= 1)  // (one halving more than nrows - r0 rows need at most)
 #pragma unroll
             for (uint32_t u = 0; u < PER; ++u)
                 if (hi[u] - lo[u] > 1) {
@@ -269,12 +290,6 @@ __global__ void __launch_bounds__(kThreads)
             if (k < e && k >= rows_b && k < rows_e) __stcs(ro + k, lo[u]);
         }
         return;
-    }
-    // rows after the first that start inside the run (empty ones share a
-    // position with the next: the largest stays)
-    for (uint32_t r = r0 + 1 + t; r <= r1; r += kThreads) {
-        const uint32_t at = __ldg(rp + r);
-        if (at >= b && at < e) atomicMax(&mark[at - b], r);
     }
     __syncthreads();
     uint32_t v[PER], m = 0;
@@ -452,11 +467,11 @@ clsparseStatus coo2csr(const clsparseCooMatrix* coo, clsparseCsrMatrix* csr, cls
     const uint32_t nnz = static_cast<uint32_t>(coo->num_nonzeros), nrows = static_cast<uint32_t>(coo->num_rows);
     uint32_t* rp = dev_ptr<uint32_t>(csr->row_pointer, csr->off_row_pointer);
     if (nnz) {
-        const uint32_t runs = (nnz - 1) / kChunk + 1;
-        coo_to_csr_kernel<T><<<runs + nrows / kGapCta + 1, kThreads, 0, s>>>(
+        const uint32_t runs = (nnz - 1) / kChunk + 1, gap_ctas = nrows / kGapCta + 1;
+        coo_to_csr_kernel<T><<<runs + gap_ctas, kThreads, 0, s>>>(
             dev_ptr<const uint32_t>(coo->row_indices, coo->off_row_indices),
             dev_ptr<const uint32_t>(coo->col_indices, coo->off_col_indices),
-            dev_ptr<const T>(coo->values, coo->off_values), nnz, nrows, runs, rp,
+            dev_ptr<const T>(coo->values, coo->off_values), nnz, nrows, gap_ctas, rp,
             dev_ptr<uint32_t>(csr->col_indices, csr->off_col_indices), dev_ptr<T>(csr->values, csr->off_values));
     } else {
         fill_u32_kernel<<<grid_for(static_cast<uint64_t>(nrows) + 1, control->sm_count), kThreads, 0, s>>>(

@@ -69,7 +69,8 @@ __global__ void __launch_bounds__(SHORT ? kThreadsShort : kThreads)
                  const T* __restrict__ beta_p, const T* __restrict__ B, DenseView bv, T* __restrict__ C,
                  DenseView cv) {
     using V = Vec<T, VW>;
-    if constexpr (G == 1) L = 1;
+    constexpr uint32_t NT = SHORT ? kThreadsShort : kThreads;
+    if constexpr (SHORT && G == 1) L = 1;
     const T alpha = *alpha_p, beta = *beta_p;
     const uint32_t lane = threadIdx.x & (G - 1);
     // Groups of one warp may be at different rows and iterations: shuffles
@@ -77,13 +78,14 @@ __global__ void __launch_bounds__(SHORT ? kThreadsShort : kThreads)
     const unsigned mask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31u) & ~(G - 1u)));
     const uint32_t S = G / L;  // >= 1: L <= G
     const uint32_t slot = lane / L, v = lane - slot * L;
-    const uint64_t group = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / G;
-    const uint64_t ngroups = static_cast<uint64_t>(gridDim.x) * blockDim.x / G;
+    const uint64_t group = (static_cast<uint64_t>(blockIdx.x) * NT + threadIdx.x) / G;
+    const uint64_t ngroups = static_cast<uint64_t>(gridDim.x) * NT / G;
     const uint64_t work = static_cast<uint64_t>(nrows) * tiles;
     for (uint64_t w = group; w < work; w += ngroups) {
-        // (one tile, the usual case, without the division)
-        const uint32_t row = static_cast<uint32_t>(tiles == 1 ? w : w / tiles);
-        const uint32_t vec = tiles == 1 ? v : static_cast<uint32_t>(w - static_cast<uint64_t>(row) * tiles) * L + v;
+        // (short rows: one tile, the usual case, without the division)
+        const bool one = SHORT && tiles == 1;
+        const uint32_t row = static_cast<uint32_t>(one ? w : w / tiles);
+        const uint32_t vec = one ? v : static_cast<uint32_t>(w - static_cast<uint64_t>(row) * tiles) * L + v;
         const bool on = slot < S && vec < nvec;
         const T* Bc = B + static_cast<size_t>(vec) * VW * bv.cs;
         const uint32_t rb = dev::ld_ro(rp + row), re = dev::ld_ro(rp + row + 1);
