@@ -1,6 +1,6 @@
 """The banded inner solves of the mixed-precision refinement (diagonal
-storage, one fused cooperative launch per inner solve; clsparse_b200/csrc/
-dia.cu) against the CSR inner solves they replace (CLSPARSE_B200_DIA=0),
+storage, one fused cooperative launch per inner solve, on chip and streamed;
+clsparse_b200/csrc/dia.cu, dia_resident.cu) against the CSR inner solves they replace (CLSPARSE_B200_DIA=0),
 through the C ABI.
 
 Both must reach the FP64 residual 1e-10 (recomputed on the host) and agree
@@ -19,6 +19,16 @@ from clsparse_b200 import _lib as L
 from clsparse_b200 import api, learn, matgen
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True, params=["onchip", "streamed"])
+def form(request, monkeypatch):
+    """Every test with the inner solves on chip and with them streaming; the
+    engine they are to run on."""
+    if request.param == "streamed":
+        monkeypatch.setenv("CLSPARSE_B200_DIA_RESIDENT", "0")
+        return "banded"
+    return "banded-on-chip"
 
 
 def residual(rp, col, val, x, b):
@@ -48,11 +58,12 @@ CASES = {
 @pytest.mark.parametrize("precond", [L.DIAGONAL, L.NOPRECOND], ids=["jacobi", "none"])
 @pytest.mark.parametrize("inner", ["fp32", "bf16"])
 @pytest.mark.parametrize("case", sorted(CASES))
-def test_banded_mixed_matches_csr(ctrl, orc, monkeypatch, case, inner, precond):
+def test_banded_mixed_matches_csr(ctrl, orc, monkeypatch, form, case, inner, precond):
     mat = CASES[case]()
     n = len(mat[0]) - 1
     b = np.random.default_rng(3).uniform(-1, 1, n)
     xb, ib = mixed(ctrl, mat, b, inner, True, monkeypatch, precond)
+    assert ctrl.solver_engine() == form
     xc, ic = mixed(ctrl, mat, b, inner, False, monkeypatch, precond)
     xo, _ = orc.solve("cg", np.float64, *mat, np.zeros(n), b, L.DIAGONAL, 100000, 1e-13, 0.0)
     if inner == "bf16":
@@ -97,11 +108,13 @@ def test_banded_learned_matches_csr(ctrl, monkeypatch):
 
 
 @pytest.mark.parametrize("m", [96, 300])
-def test_local_t_form_equals_three_phase_form(ctrl, monkeypatch, m):
-    """The learned iteration with t = G r kept per CTA in shared memory (two
+def test_local_t_form_equals_three_phase_form(ctrl, monkeypatch, form, m):
+    """The streamed learned iteration with t = G r kept per CTA in shared memory (two
     grid exchanges per iteration) computes every value the three-phase form
     computes, in the same order: the solves agree bit for bit. 300^2 rows
     gives slices whose halo reaches into the next CTA's rows."""
+    if form != "banded":
+        pytest.skip("on chip t is always kept")
     spai, _ = learn.train(ctrl, sizes=(32,), seeds=range(2), steps=40, lr=3e-3)
     smp = learn.Sample(ctrl, m, 7, with_probes=False)
     spai.set_matrix(smp.A, ctrl)

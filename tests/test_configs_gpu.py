@@ -5,9 +5,9 @@ oracle.
   reference's L1 stop test at 1e-10 (clsparseDcsrcg), against the serial
   oracle restatement of the reference CG (conjugate-gradients.hpp:47-228):
   the same stop decision within 1% of the iterations, the same initial
-  residual, and the same solution -- on the default engine and on the banded
-  drop-in engine (solver loop mode 3), which also runs the FP64 Jacobi-CG of
-  C3 and C5.
+  residual, and the same solution -- on the graph engine and on the banded
+  drop-in engine (solver loop mode 3; the default, too, at these sizes), as
+  the FP64 Jacobi-CG of C3 and C5.
 * C3 -- 3D 7-point log-normal diffusion 128^3 (2,097,152 rows, sigma 1.5)
   and C5 -- 2D Gaussian-random-field diffusion 1024^2 (1,048,576 rows,
   correlation length 0.05, sigma 2): FP64 Jacobi-CG, the mixed-precision
@@ -100,8 +100,15 @@ def c1_oracle_cg():
     return oracle.solve("cg", np.float64, rp, col, val, np.zeros(n), rhs(n), L.DIAGONAL, 200000, 1e-10, 0.0)
 
 
+def engine_for(monkeypatch, loop_mode):
+    """The graph engine for loop mode 0 (the banded one switched off)."""
+    if loop_mode == 0:
+        monkeypatch.setenv("CLSPARSE_B200_DIA", "0")
+
+
 @pytest.mark.parametrize("loop_mode", [0, 3], ids=["graph", "banded"])
-def test_c1_poisson512_cg_matches_oracle(ctrl, orc, loop_mode):
+def test_c1_poisson512_cg_matches_oracle(ctrl, orc, monkeypatch, loop_mode):
+    engine_for(monkeypatch, loop_mode)
     rp, col, val = config("C1")
     n = len(rp) - 1
     b = rhs(n)
@@ -111,6 +118,7 @@ def test_c1_poisson512_cg_matches_oracle(ctrl, orc, loop_mode):
     info = api.solve("cg", x, A, bt, sc, ctrl)
     sc.release()
     ctrl.set_solver_loop_mode(0)
+    assert ctrl.solver_engine() == ("graph" if loop_mode == 0 else "banded-on-chip")
     xo, oi = c1_oracle_cg()
     assert oi.nIters > 1000
     assert abs(info["nIters"] - oi.nIters) <= max(3, int(0.01 * oi.nIters)), (info, oi.nIters)
@@ -135,8 +143,10 @@ def _fp64_cg(ctrl, name, loop_mode=0):
 
 @pytest.mark.parametrize("loop_mode", [0, 3], ids=["graph", "banded"])
 @pytest.mark.parametrize("name", ["C3", "C5"])
-def test_fp64_jacobi_cg_at_config_matches_oracle(ctrl, orc, name, loop_mode):
+def test_fp64_jacobi_cg_at_config_matches_oracle(ctrl, orc, monkeypatch, name, loop_mode):
+    engine_for(monkeypatch, loop_mode)
     xs, info = _fp64_cg(ctrl, name, loop_mode)
+    assert ctrl.solver_engine() == ("graph" if loop_mode == 0 else "banded-on-chip" if name == "C5" else "banded")
     # the oracle's threaded CG to the same L2 tolerance: same iteration count
     # up to reduction order
     it_o = oracle_iterations_1e10(name)

@@ -1,6 +1,6 @@
 """The drop-in clsparse{S,D}csrcg and clsparse{S,D}csrbicgStab on the banded
-engine (solver loop mode 3) against the oracle restatements of the
-reference CG and BiCGStab (src/library/solvers/conjugate-gradients.hpp:73-226,
+engine (solver loop mode 3), with the vectors on chip and streamed through L2,
+against the oracle restatements of the reference CG and BiCGStab (src/library/solvers/conjugate-gradients.hpp:73-226,
 biconjugate-gradients-stabilized.hpp:61-266).
 
 Parity bar as for the other loop modes: the same stop decision (iteration
@@ -26,6 +26,16 @@ from clsparse_b200 import api, matgen
 pytestmark = pytest.mark.gpu
 
 NP = {torch.float64: np.float64, torch.float32: np.float32}
+
+
+@pytest.fixture(autouse=True, params=["onchip", "streamed"])
+def form(request, monkeypatch):
+    """Every test with the solves on chip and with them streaming; the engine a
+    banded solve is to run on."""
+    if request.param == "streamed":
+        monkeypatch.setenv("CLSPARSE_B200_DIA_RESIDENT", "0")
+        return "banded"
+    return "banded-on-chip"
 
 
 def banded9(n: int, seed: int = 4):
@@ -60,7 +70,15 @@ PROBLEMS = {
 }
 
 
-def run(ctrl, rp, col, val, x0, b, dtype, precond, max_iters, rel, abs_, loop_mode=3, sc=None, norm=0, kind="cg"):
+def run(ctrl, rp, col, val, x0, b, dtype, precond, max_iters, rel, abs_, loop_mode=3, sc=None, norm=0, kind="cg",
+        graph=None):
+    """graph (a monkeypatch): on the graph engine, the banded one switched off."""
+    if graph is not None:
+        with graph.context() as m:
+            m.setenv("CLSPARSE_B200_DIA", "0")
+            out = run(ctrl, rp, col, val, x0, b, dtype, precond, max_iters, rel, abs_, 0, sc, norm, kind)
+        assert ctrl.solver_engine() == "graph"
+        return out
     ctrl.set_solver_loop_mode(loop_mode)
     A = api.CsrMatrix.from_numpy(rp, col, val, dtype=dtype)
     A.create_meta(ctrl)
@@ -88,13 +106,14 @@ def l1_residual(rp, col, val, x, b):
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
 @pytest.mark.parametrize("precond", [L.DIAGONAL, L.NOPRECOND], ids=["jacobi", "none"])
 @pytest.mark.parametrize("prob", sorted(PROBLEMS))
-def test_banded_cg_matches_oracle(ctrl, orc, prob, precond, dtype):
+def test_banded_cg_matches_oracle(ctrl, orc, form, prob, precond, dtype):
     rp, col, val = PROBLEMS[prob]()
     n = len(rp) - 1
     b = np.random.default_rng(1).uniform(-1, 1, n)
     rel = 1e-10 if dtype == torch.float64 else 1e-5
     t = NP[dtype]
     x, info, status = run(ctrl, rp, col, val, np.zeros(n), b, dtype, precond, 5000, rel, 0.0)
+    assert ctrl.solver_engine() == ("graph" if prob == "random_spd" else form)
     _, oi = orc.solve("cg", t, rp, col, val, np.zeros(n, t), np.asarray(b, t), precond, 5000, rel, 0.0)
     slack = max(3, int(0.03 * oi.nIters))
     assert abs(info["nIters"] - oi.nIters) <= slack, (info, oi.nIters)
@@ -106,12 +125,12 @@ def test_banded_cg_matches_oracle(ctrl, orc, prob, precond, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
-def test_banded_cg_agrees_with_graph_engine(ctrl, dtype):
+def test_banded_cg_agrees_with_graph_engine(ctrl, monkeypatch, dtype):
     rp, col, val = matgen.diffusion3d_lognormal(20, sigma=1.5, seed=7)
     n = len(rp) - 1
     b = np.random.default_rng(5).uniform(-1, 1, n)
     rel = 1e-10 if dtype == torch.float64 else 1e-5
-    xg, ig, _ = run(ctrl, rp, col, val, np.zeros(n), b, dtype, L.DIAGONAL, 5000, rel, 0.0, loop_mode=0)
+    xg, ig, _ = run(ctrl, rp, col, val, np.zeros(n), b, dtype, L.DIAGONAL, 5000, rel, 0.0, graph=monkeypatch)
     xb, ib, _ = run(ctrl, rp, col, val, np.zeros(n), b, dtype, L.DIAGONAL, 5000, rel, 0.0, loop_mode=3)
     assert abs(ig["nIters"] - ib["nIters"]) <= max(3, int(0.03 * ig["nIters"]))
     assert ib["initialResidual"] == pytest.approx(ig["initialResidual"], rel=1e-6)
@@ -119,12 +138,12 @@ def test_banded_cg_agrees_with_graph_engine(ctrl, dtype):
     assert np.abs(xb - xg).max() <= tol * np.abs(xg).max()
 
 
-def test_banded_cg_l2_norm_option(ctrl, orc):
+def test_banded_cg_l2_norm_option(ctrl, orc, monkeypatch):
     rp, col, val = matgen.poisson2d(50)
     n = len(rp) - 1
     b = np.random.default_rng(8).uniform(-1, 1, n)
     xg, ig, _ = run(ctrl, rp, col, val, np.zeros(n), b, torch.float64, L.DIAGONAL, 3000, 1e-9, 0.0,
-                    loop_mode=0, norm=1)
+                    norm=1, graph=monkeypatch)
     xb, ib, _ = run(ctrl, rp, col, val, np.zeros(n), b, torch.float64, L.DIAGONAL, 3000, 1e-9, 0.0,
                     loop_mode=3, norm=1)
     assert abs(ig["nIters"] - ib["nIters"]) <= 3
@@ -191,7 +210,7 @@ def test_banded_cg_exact_initial_guess(ctrl):
     np.testing.assert_array_equal(x, xs)
 
 
-def test_banded_cg_missing_diagonal_runs_graph_engine(ctrl):
+def test_banded_cg_missing_diagonal_runs_graph_engine(ctrl, monkeypatch):
     """Row 1 without a diagonal entry under Jacobi: the banded engine leaves x
     untouched and the graph engine reports the missing diagonal as in the
     other loop modes."""
@@ -200,8 +219,9 @@ def test_banded_cg_missing_diagonal_runs_graph_engine(ctrl):
     col[2:4] = [0, 2]
     n = 3
     _, _, s3 = run(ctrl, rp, col, np.abs(val) + 1, np.zeros(n), np.ones(n), torch.float64, L.DIAGONAL, 5, 1e-12, 0.0)
+    assert ctrl.solver_engine() == "graph"
     _, _, s0 = run(ctrl, rp, col, np.abs(val) + 1, np.zeros(n), np.ones(n), torch.float64, L.DIAGONAL, 5, 1e-12, 0.0,
-                   loop_mode=0)
+                   graph=monkeypatch)
     assert s3 & 1 and s3 == s0
 
 
@@ -263,8 +283,9 @@ def convdiff5(m: int = 40):
 def test_banded_cg_symmetric_form_is_bitwise_equal(ctrl, monkeypatch, prob, dtype):
     """The form that reads a symmetric matrix's lower diagonals from the upper
     ones (forced on; by default it runs only when the working set exceeds half
-    of L2) gives the same x bit for bit; a non-symmetric matrix, or one with
-    more diagonals than the form takes, runs the plain form."""
+    of L2, or the chip does not hold every diagonal) gives the same x bit for
+    bit; a non-symmetric matrix, or one with more diagonals than the streaming
+    form takes, runs the plain form."""
     rp, col, val = {"poisson64": lambda: matgen.poisson2d(64), "tridiag": lambda: tridiag(5000),
                     "convdiff5": convdiff5,
                     "diffusion3d": lambda: matgen.diffusion3d_lognormal(16, sigma=1.0, seed=2)}[prob]()
@@ -294,13 +315,14 @@ def bicg_slack(n_ref):
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
 @pytest.mark.parametrize("precond", [L.DIAGONAL, L.NOPRECOND], ids=["jacobi", "none"])
 @pytest.mark.parametrize("prob", sorted(BICG_PROBLEMS))
-def test_banded_bicgstab_matches_oracle(ctrl, orc, prob, precond, dtype):
+def test_banded_bicgstab_matches_oracle(ctrl, orc, form, prob, precond, dtype):
     rp, col, val = BICG_PROBLEMS[prob]()
     n = len(rp) - 1
     b = np.random.default_rng(1).uniform(-1, 1, n)
     rel = 1e-10 if dtype == torch.float64 else 1e-5
     t = NP[dtype]
     x, info, status = run(ctrl, rp, col, val, np.zeros(n), b, dtype, precond, 5000, rel, 0.0, kind="bicgstab")
+    assert ctrl.solver_engine() == ("graph" if prob == "random_spd" else form)
     _, oi = orc.solve("bicgstab", t, rp, col, val, np.zeros(n, t), np.asarray(b, t), precond, 5000, rel, 0.0)
     assert abs(info["nIters"] - oi.nIters) <= bicg_slack(oi.nIters), (info, oi.nIters)
     assert info["initialResidual"] == pytest.approx(oi.initialResidual, rel=1e-5)
@@ -311,13 +333,13 @@ def test_banded_bicgstab_matches_oracle(ctrl, orc, prob, precond, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32], ids=["f64", "f32"])
-def test_banded_bicgstab_agrees_with_graph_engine(ctrl, dtype):
+def test_banded_bicgstab_agrees_with_graph_engine(ctrl, monkeypatch, dtype):
     rp, col, val = convdiff5(64)
     n = len(rp) - 1
     b = np.random.default_rng(5).uniform(-1, 1, n)
     rel = 1e-10 if dtype == torch.float64 else 1e-5
-    xg, ig, _ = run(ctrl, rp, col, val, np.zeros(n), b, dtype, L.DIAGONAL, 5000, rel, 0.0, loop_mode=0,
-                    kind="bicgstab")
+    xg, ig, _ = run(ctrl, rp, col, val, np.zeros(n), b, dtype, L.DIAGONAL, 5000, rel, 0.0, kind="bicgstab",
+                    graph=monkeypatch)
     xb, ib, _ = run(ctrl, rp, col, val, np.zeros(n), b, dtype, L.DIAGONAL, 5000, rel, 0.0, loop_mode=3,
                     kind="bicgstab")
     assert abs(ig["nIters"] - ib["nIters"]) <= bicg_slack(ig["nIters"])
@@ -396,7 +418,7 @@ def test_banded_bicgstab_barrier_timeout_is_reported_and_recovers(ctrl, orc, mon
     assert l1_residual(rp, col, val, x, b) <= 1e-9
 
 
-def test_default_bicgstab_counts_are_as_close_to_the_oracle_as_the_graph_engines(ctrl, orc, monkeypatch):
+def test_default_bicgstab_counts_are_as_close_to_the_oracle_as_the_graph_engines(ctrl, orc, form, monkeypatch):
     """Above 2048 rows the default mode's BiCGStab runs on the banded engine.
     The iteration count of a run depends on the order of the sums on any engine
     (on average 2.4 % from the oracle here, 2.9 % on the graph engine; within 5 % and
@@ -421,7 +443,7 @@ def test_default_bicgstab_counts_are_as_close_to_the_oracle_as_the_graph_engines
                     monkeypatch.setenv("CLSPARSE_B200_DIA", env)
                     _, info, _ = run(ctrl, rp, col, val, np.zeros(n), b, dtype, L.DIAGONAL, 5000, rel, 0.0,
                                      loop_mode=0, kind="bicgstab")
-                    assert ctrl.solver_engine() == ("banded-on-chip" if engine == "banded" else "graph")
+                    assert ctrl.solver_engine() == (form if engine == "banded" else "graph")
                     assert info["currentResidual"] <= rel
                     off[engine].append(abs(info["nIters"] - oi.nIters) / oi.nIters)
     mean = {k: float(np.mean(v)) for k, v in off.items()}

@@ -1,6 +1,6 @@
 """The banded solves with their vectors on chip against the same solves
-streaming their vectors through L2 (CLSPARSE_B200_DIA_RESIDENT=0), which the
-other tests pin to the oracle and to the reference's runs. Both form every
+streaming their vectors through L2 (CLSPARSE_B200_DIA_RESIDENT=0), which
+test_dia_cg_gpu.py and test_banded_gpu.py hold to the oracle and to CSR. Both form every
 row and vector entry with the same operations; only the FP64 sums of the dot
 products run in another order. A fixed, small number of iterations from the
 same start therefore agrees to rounding: the scalars differ by a few 1e-16 (FP64
@@ -10,9 +10,10 @@ carries that over with a factor below ten for these matrices (condition below
 2^-24 after the sum, so an iterate moves by at most a few 1e-6.
 
 Sizes: one row to a few, around one CTA's share (1024 rows), around the
-register arrays (4, 14 and 28 rows per thread of 512 on 148 SMs), odd splits;
+register arrays (2, 4 and 14 rows per thread of 512 on 148 SMs), odd splits;
 stencils within a CTA, across neighbours, and across several CTAs (the plain
-exchange of z); 3 to 9 diagonals and padded counts."""
+exchange of z); 3 to 9 diagonals and padded counts. Just beyond what the chip
+takes (rows, halo, shared memory) both sides stream, as asserted."""
 from __future__ import annotations
 
 import threading
@@ -57,13 +58,27 @@ def both(monkeypatch, fn):
 
 
 SMALL = [(1, [1]), (2, [1]), (3, [1, 2]), (40, [1, 7]), (1023, [1, 31]), (1024, [1, 32]), (1025, [1, 32, 900]),
-         (2049, [1, 2, 3, 4]), (5000, [1, 2100]), (12345, [1, 20, 400]), (30011, [1, 9000])]
+         (2049, [1, 2, 3, 4]), (5000, [1, 2100]), (12345, [1, 20, 400]), (30011, [1, 7000]), (30011, [1, 9000])]
 LARGE = [(303104, [1, 551]), (303105, [1, 551]), (200001, [1, 60, 3600]), (262144, [1, 512])]
 HUGE = [(1060864, [1, 1030]), (1060865, [1, 1030]), (1000000, [1, 100, 10000])]
 
 
 def _case_id(c):
     return f"n{c[0]}o{c[1][-1]}"
+
+
+def expected_engine(kind, case, dtype):
+    """On chip, but for a halo wider than it pays (18,000 rows), more than 7168
+    (CG) or 2048 (BiCGStab) rows a CTA, and BiCGStab halos beyond the shared
+    memory (five words a halo row). A single row is no STREAM block of its
+    meta: the graph engine's."""
+    n, offs = case
+    if n == 1:
+        return "graph"
+    if offs[-1] == 9000 or n > 1060864:
+        return "banded"
+    wide = 5 * 2 * offs[-1] * (8 if dtype == torch.float64 else 4) > 220000
+    return "banded" if kind == "bicgstab" and (n > 303104 or wide) else "banded-on-chip"
 
 
 @pytest.mark.parametrize("precond", [L.DIAGONAL, L.NOPRECOND], ids=["jacobi", "none"])
@@ -87,9 +102,12 @@ def test_dropin_solves(ctrl, monkeypatch, case, kind, dtype, precond):
         sc = api.SolverControl(precond, iters, tol, 0.0)
         info = api.solve(kind, x, A, b, sc, ctrl)
         sc.release()
+        engines.append(ctrl.solver_engine())
         return x.double().cpu().numpy(), info
 
+    engines = []
     (x, i), (xr, ir) = both(monkeypatch, lambda: solve(12 if n > 64 else 2, 0.0))
+    assert engines == [expected_engine(kind, case, dtype), "graph" if n == 1 else "banded"]
     tol = 1e-9 if dtype == torch.float64 else 2e-4
     if n > 64:
         assert i["nIters"] == ir["nIters"]
@@ -105,9 +123,10 @@ def test_dropin_solves(ctrl, monkeypatch, case, kind, dtype, precond):
 
 
 @pytest.mark.parametrize("inner", ["fp32", "bf16"])
-@pytest.mark.parametrize("case", [(50, [1, 7]), (1025, [1, 32]), (30011, [1, 9000]), (20000, [1, 2, 3, 4]),
-                                  (303105, [1, 551]), (1060865, [1, 80, 6400]), (2121728, [1, 128, 16384]),
-                                  (2121729, [1, 1456])], ids=_case_id)
+@pytest.mark.parametrize("case", [(50, [1, 7]), (1025, [1, 32]), (30011, [1, 6000]), (30011, [1, 9000]),
+                                  (20000, [1, 2, 3, 4]), (303105, [1, 551]), (1060864, [1, 80, 6400]),
+                                  (1060865, [1, 80, 6400]), (2121728, [1, 128, 16384]), (2121729, [1, 1456])],
+                         ids=_case_id)
 def test_inner_solves(ctrl, monkeypatch, case, inner):
     """The refinement's inner PCG: the same number of refinements, and the FP64
     true residual recomputed here meets the tolerance on both."""
@@ -122,11 +141,14 @@ def test_inner_solves(ctrl, monkeypatch, case, inner):
         sc = api.SolverControl(L.DIAGONAL, 20000, 1e-10, 0.0)
         info = api.cg_mixed(x, A, b, sc, ctrl, inner=inner, inner_tol=0.1)
         sc.release()
+        engines.append(ctrl.solver_engine())
         return x.cpu().numpy(), info
 
+    engines = []
     M = sp.csr_matrix((val, col.astype(np.int64), rp.astype(np.int64)), shape=(n, n))
     bb = b.cpu().numpy()
     (x, i), (xr, ir) = both(monkeypatch, solve)
+    assert engines == [expected_engine("cg", case, torch.float32), "banded"]
     for v, info in ((x, i), (xr, ir)):
         assert info["converged"] == 1
         assert np.linalg.norm(bb - M @ v) <= 1.5e-10 * np.linalg.norm(bb)
@@ -159,9 +181,12 @@ def test_learned_inner_solves(ctrl, monkeypatch, shape):
         sc = api.SolverControl(L.DIAGONAL, 60000 if len(shape) == 1 else 200, 1e-9, 0.0)
         info = api.cg_learned(x, A, b, sc, spai, ctrl, inner="fp32", inner_tol=0.3)
         sc.release()
+        engines.append(ctrl.solver_engine())
         return x.cpu().numpy(), info
 
+    engines = []
     (x, i), (xr, ir) = both(monkeypatch, solve)
+    assert engines == ["banded-on-chip", "banded"]
     spai.release()
     M = sp.csr_matrix((val, col.astype(np.int64), rp.astype(np.int64)), shape=(n, n))
     bb = b.cpu().numpy()

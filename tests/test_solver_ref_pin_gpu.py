@@ -4,9 +4,9 @@ reference's OWN kernels (tests/golden/solvers_ref.npz): the reference's
 solver-test settings (src/tests/test-solvers.cpp:267-277) and a tighter set,
 FP64 and FP32, Jacobi and no preconditioner, a matrix without a meta
 (the reference test's csrmv_general path) and with one (csrmv_adaptive).
-Every run also goes through the persistent engine and the banded loop mode
-(CG and BiCGStab on the stencil matrices with a meta; the other runs fall
-through to the graph engine). The bars are stated in
+Every run goes through the default mode (CG on the stencil matrices with a
+meta on the banded engine, the rest on the graph engine), the graph engine, the
+persistent engine and the banded loop mode (BiCGStab on those matrices, too). The bars are stated in
 tests/solver_golden.py; the library's reductions sum in a different order
 from the reference's, as two GPUs would."""
 from __future__ import annotations
@@ -47,12 +47,17 @@ def lib_solve(ctrl, run, loop_mode, history=False):
     return x.cpu().numpy().astype(np.float64), info, (rel, abs_, max_it)
 
 
-@pytest.mark.parametrize("loop_mode", [0, 2, 3], ids=["graph", "persistent", "banded"])
+@pytest.mark.parametrize("engine,loop_mode", [("default", 0), ("graph", 0), ("persistent", 2), ("banded", 3)],
+                         ids=["default", "graph", "persistent", "banded"])
 @pytest.mark.parametrize("run", RUNS, ids=[G.run_id(r) for r in RUNS])
-def test_library_solver_matches_reference_run(ctrl, run, loop_mode):
+def test_library_solver_matches_reference_run(ctrl, monkeypatch, run, engine, loop_mode):
     name, setting, method, t, pre, path = run
+    if engine == "graph":
+        monkeypatch.setenv("CLSPARSE_B200_DIA", "0")
     xr, it, init, cur, hist = G.reference(D, run)
     x, info, (rel, abs_, max_it) = lib_solve(ctrl, run, loop_mode)
+    if engine == "graph":
+        assert ctrl.solver_engine() == "graph"
     assert abs(info["nIters"] - it) <= G.iter_slack(method, t, it, banded=loop_mode == 3), (info, it)
     assert info["initialResidual"] == pytest.approx(init, rel=1e-12 if t == "d" else 1e-6)
     c = info["currentResidual"]

@@ -1,6 +1,8 @@
 """CG / BiCGStab through the C ABI against the oracle restatement of the
 reference solvers (src/library/solvers/conjugate-gradients.hpp,
-biconjugate-gradients-stabilized.hpp).
+biconjugate-gradients-stabilized.hpp), on the graph, host-chunk and persistent
+engines: the banded engine, which the default modes take on the stencil
+matrices, is switched off here (test_dia_cg_gpu.py, test_resident_gpu.py).
 
 Parity bar: the same stop decision (iteration counts within a small slack --
 the GPU sums reductions in a different order), the reported residuals agree,
@@ -17,6 +19,11 @@ from clsparse_b200 import api, matgen
 pytestmark = pytest.mark.gpu
 
 NP = {torch.float64: np.float64, torch.float32: np.float32}
+
+
+@pytest.fixture(autouse=True)
+def no_banded_engine(monkeypatch):
+    monkeypatch.setenv("CLSPARSE_B200_DIA", "0")
 
 
 def run(ctrl, kind, rp, col, val, x0, b, dtype, precond, max_iters, rel, abs_, meta=True, loop_mode=0):
@@ -59,6 +66,7 @@ def test_solver_parity(ctrl, orc, kind, prob, precond, dtype, loop_mode):
     rel = 1e-10 if dtype == torch.float64 else 1e-5
     t = NP[dtype]
     x, info, _ = run(ctrl, kind, rp, col, val, np.zeros(n), b, dtype, precond, 5000, rel, 0.0, loop_mode=loop_mode)
+    assert ctrl.solver_engine() == ("persistent" if loop_mode == 2 and kind == "cg" else "graph")
     xo, oi = orc.solve(kind, t, rp, col, val, np.zeros(n, t), np.asarray(b, t), precond, 5000, rel, 0.0)
     # BiCGStab's convergence history is irregular and reacts to the order of
     # the reduction sums; CG's is smooth.
@@ -77,8 +85,10 @@ def test_solver_loop_modes_agree(ctrl, kind):
     b = np.random.default_rng(5).uniform(-1, 1, n)
     x0, i0, _ = run(ctrl, kind, rp, col, val, np.zeros(n), b, torch.float64, L.DIAGONAL, 3000, 1e-9, 0.0,
                     loop_mode=0)
+    assert ctrl.solver_engine() == "graph"
     x1, i1, _ = run(ctrl, kind, rp, col, val, np.zeros(n), b, torch.float64, L.DIAGONAL, 3000, 1e-9, 0.0,
                     loop_mode=1)
+    assert ctrl.solver_engine() == "chunks"
     assert i0 == i1
     assert np.array_equal(x0, x1)
 
