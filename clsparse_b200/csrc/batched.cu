@@ -15,8 +15,9 @@
 // are solved by the resident kernel (batched_resident.cuh), one launch per
 // cluster size on streams of their own, the largest systems first.
 //
-// The others run in the persistent general kernel: one CTA per resident slot
-// takes the next system from a device work queue (largest first). When all of
+// The others run in the persistent general kernel (a cliff: 52,900 rows take 6 us
+// an iteration on eight SMs, 67,600 rows, which do not fit, 116 on one CTA here):
+// one CTA per resident slot takes the next system from a device work queue (largest first). When all of
 // them are banded (systems too large for a cluster's shared memory), their
 // products come from a per-system diagonal-storage copy laid out at every
 // call: one thread per row, the values and the vector entries independent

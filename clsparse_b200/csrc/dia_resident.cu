@@ -38,9 +38,12 @@
 namespace clsp {
 namespace {
 
-// Threads of a CTA, one CTA per SM: 128 registers a thread, which hold 14 rows
-// of x, r and q in FP64. (1024 threads of 64 registers measured slower in FP32:
-// 6.6 us an iteration instead of 5.3 on 512^2, no change on 100^3.)
+// Threads of a CTA, one CTA per SM: 128 registers a thread. 14 rows of x, r and q
+// take 84 of them in FP64, and those CG kernels (more than 2048 rows a CTA: from
+// 303,105 rows on 148 SMs) store 200 to 340 bytes of others to the stack; FP64
+// BiCGStab with four rows stores up to 184, FP32 kernels at most 64. (1024 threads
+// of 64 registers measured slower in FP32: 6.6 us an iteration instead of 5.3 on
+// 512^2, no change on 100^3.)
 constexpr int kResThreads = 512;
 constexpr int kFewRows = kResidentBicgRows / kResThreads;   // rows per thread the kernels are built for: 4,
 constexpr int kManyRows = kResidentCgRows / kResThreads;    // 14
@@ -1044,8 +1047,12 @@ cudaError_t pcg_launch(DiaPcgResidentArgs<VA, VG>& args, cudaStream_t s) {
 }
 
 // Rows per CTA a solve aims at. An exchange costs more the more CTAs take part
-// (each polls every other's words: 0.4 us with 2, 0.9 with 19, 1.5 with 148,
-// bare), so a small system runs on fewer SMs.
+// (each polls every other's words: 0.4 us bare with 2, 1.0 with 148), a CTA's own
+// sums and products more the more rows it has. CG, FP64, us an iteration with
+// 256, 512, 1024 and 2048 rows a CTA: 64^2 4.2, 3.7, 3.8, 4.4; 100^2 4.5, 4.5, 4.0,
+// 4.4; 200^2 5.4, 4.3, 4.4, 5.1; 24^3 5.4, 5.7, 6.1, 6.5; 40^3 6.0, 5.9, 6.1, 7.3;
+// BiCGStab 200^2 7.8, 7.5, 7.7, 9.5. (From 152,000 rows on every SM takes part
+// either way.)
 constexpr uint32_t kRowsPerCta = 1024;
 
 // The part of a plan common to all methods: grid, rows, halo.

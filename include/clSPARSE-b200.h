@@ -135,7 +135,9 @@ typedef struct clsparseB200BatchResult_
  * systemOffsets a host array of numSystems+1 entries starting at 0 and ending
  * at num_rows) with Jacobi-CG in FP32: banded systems (at most 8 column offsets)
  * of up to about 57,000 rows are held on chip, each by a cluster of up to 8
- * SMs, the others share one persistent launch. Each system stops when its FP64 true residual
+ * SMs, the others share one persistent launch, one CTA for each (52,900 rows
+ * take 6 us an iteration, 67,600 rows 116). clsparseOutOfResources leaves x as it
+ * was. Each system stops when its FP64 true residual
  * ||b - A x||_2 / ||b||_2 <= the control's relTol (checked whenever the FP32
  * recursive residual says so; CG restarts from x otherwise) or after maxIters
  * iterations. lanesPerRow (optional, per system: 1..32, a power of two) sets
