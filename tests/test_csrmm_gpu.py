@@ -153,9 +153,8 @@ def test_csrmm_vector_widths(ctrl, dtype, ncols, pad, off):
 @pytest.mark.parametrize("ncols", [1, 2, 3, 4, 8, 16, 31, 32, 33, 65, 100])
 def test_csrmm_short_rows(ctrl, dtype, ncols, major):
     """The form for rows of fewer than 8 nonzeros on average: every remainder of
-    its 4, 2 and 1 steps, long rows among short ones, full and narrow tiles, and
-    the other form for the same matrix when a meta shows a long row. Tolerance
-    as above (at most 1500 products: the absolute sum scales)."""
+    its 4, 2 and 1 steps, long rows among short ones, full and narrow tiles.
+    Tolerance as above (at most 1500 products: the absolute sum scales)."""
     mj = L.rowMajor if major == "row" else L.columnMajor
     lens = [0, 1, 2, 3, 4, 5, 6, 7, 9, 11, 15, 17, 31, 33, 0, 0] * 6 + [1] * 400 + [1500]
     n, m = len(lens), 1600
@@ -172,15 +171,12 @@ def test_csrmm_short_rows(ctrl, dtype, ncols, major):
     a = torch.tensor([-0.75], dtype=dtype, device="cuda")
     b = torch.tensor([0.5], dtype=dtype, device="cuda")
     fn = api.lib().clsparseDcsrmm if dtype == torch.float64 else api.lib().clsparseScsrmm
-    for meta in (False, True):
-        A = api.CsrMatrix.from_numpy(rp, col, val, num_cols=m, dtype=dtype)
-        if meta:
-            A.create_meta(ctrl)
-        tb, tc = layout(B, ldb, mj, dtype), layout(C0, ldc, mj, dtype)
-        db, dc = dense(tb, m, ncols, ldb, mj), dense(tc, n, ncols, ldc, mj)
-        assert fn(C.byref(api.scalar(a)), C.byref(A.s), C.byref(db), C.byref(api.scalar(b)), C.byref(dc), ctrl.handle) == 0
-        out = unlayout(tc, n, ncols, ldc, mj)
-        assert np.max(np.abs(out - ref) / scale) <= TOL[dtype] * 10
+    A = api.CsrMatrix.from_numpy(rp, col, val, num_cols=m, dtype=dtype)
+    tb, tc = layout(B, ldb, mj, dtype), layout(C0, ldc, mj, dtype)
+    db, dc = dense(tb, m, ncols, ldb, mj), dense(tc, n, ncols, ldc, mj)
+    assert fn(C.byref(api.scalar(a)), C.byref(A.s), C.byref(db), C.byref(api.scalar(b)), C.byref(dc), ctrl.handle) == 0
+    out = unlayout(tc, n, ncols, ldc, mj)
+    assert np.max(np.abs(out - ref) / scale) <= TOL[dtype] * 10
 
 
 def test_csrmm_short_rows_are_not_slower_than_columns_one_by_one(ctrl):
