@@ -736,6 +736,7 @@ clsparseStatus prepare_cache(clsparseControl c, SolverCache& cache, const Solver
            cache.state.ensure(sizeof(SolverState<T>) + 256) != cudaSuccess) {
         cudaGetLastError();
         cache.valid = false;
+        rebuild = true;
         if (c->dia_cg == nullptr) return clsparseOutOfResources;
         c->dia_cg.reset();  // what an earlier banded solve keeps, then once more
     }
