@@ -206,12 +206,14 @@ __global__ void __launch_bounds__(kThreads)
             }
         }
     };
-#pragma unroll
-    for (uint32_t u = 0; u < PER; ++u) {
+#pragma unroll 1
+    for (uint32_t u = 0; u < PER; ++u) {  // (not unrolled, the rows read again: no code or registers more for runs without gaps)
         const uint32_t k = b + u * kThreads + threadIdx.x;
         const bool on = k < e;
-        const uint32_t from = from_of(u, k), to = to_of(u);
-        fill(on && to > from && to - from > kShortGap, from, to, k);
+        const uint32_t rk = on ? __ldg(ri + k) : 0, pk = on && k > 0 ? __ldg(ri + k - 1) : 0;
+        const uint32_t from = on && k > 0 ? (pk < nrows ? pk + 1 : nrows) : 0;
+        const uint32_t to = on ? (rk < nrows ? rk + 1 : nrows) : 0;
+        fill(to > from && to - from > kShortGap, from, to, k);
         if (e == nnz) {
             const bool last = on && k == nnz - 1;
             fill(last && to < nrows, to, nrows, nnz);
