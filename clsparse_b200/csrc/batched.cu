@@ -17,12 +17,13 @@
 //
 // The others run in the persistent general kernel (a cliff: 52,900 rows take 6 us
 // an iteration on eight SMs, 67,600 rows, which do not fit, 116 on one CTA here):
-// one CTA per resident slot takes the next system from a device work queue (largest first). When all of
-// them are banded (systems too large for a cluster's shared memory), their
-// products come from a per-system diagonal-storage copy laid out at every
-// call: one thread per row, the values and the vector entries independent
-// loads instead of the row-pointer / column-index / vector chain of CSR, and
-// rows whose whole stencil lies inside the system without clamps; otherwise
+// one CTA per resident slot takes the next system from a device work queue
+// (largest first). When all of them are banded (systems too large for a
+// cluster's shared memory), their products come from a per-system
+// diagonal-storage copy laid out at every call: one thread per row, the values
+// and the vector entries independent loads instead of the row-pointer /
+// column-index / vector chain of CSR, and rows whose whole stencil lies inside
+// the system without clamps; otherwise, and when that copy cannot be had,
 // each system's SpMV uses the lanes-per-row width the tuning table gives for
 // its size class. The kernel is held to two CTAs per SM (64 registers): the
 // diagonal loop would otherwise take 128 registers and halve the resident

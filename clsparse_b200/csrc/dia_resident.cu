@@ -1165,11 +1165,12 @@ bool resident_pcg_plan(const DiaPcgArgs<VA, VG>& a, bool learned, int sm_count, 
     if (!plan_rows(a.n, o, a.A.nd, sm_count, kResThreads, {kFewRows, kManyRows}, p)) return false;
     // Jacobi, us an inner iteration on chip / streamed, halo rows and own rows:
     // 8192 and 1024 8.0 / 8.9; 12,800 and 1024 9.3 / 9.5, and 3460 12.6 / 12.8;
-    // 16,200 and 1013 11.7 / 10.4, and 4926 14.5 / 15.5; 20,000 and 4730 15.7 /
-    // 15.0, and 6757 17.7 / 18.1. Learned (r's and q's halo beside p's): 4608 and
-    // 1024 10.1 / 11.2; 7200 and 2432 14.9 / 15.4; 8192 and 1772 14.2 / 14.2; 9800
-    // and 2318 17.8 / 16.6; 16,200 and 4926 30.2 / 23.4.
-    if (!(learned ? halo_pays(p, 7680, 2) : halo_pays(p, 12800, 7))) return false;
+    // 13,122 and 3591 12.9 / 12.8; 16,200 and 1013 11.7 / 10.4, and 4926 14.5 / 15.5;
+    // 20,000 and 4730 15.7 / 15.0, and 6757 17.7 / 18.1; 28,800 and 6811 20.3 / 18.5.
+    // Learned (r's and q's halo beside p's): 4608 and 1024 10.1 / 11.2; 7200 and
+    // 2432 14.9 / 15.4; 8192 and 1772 14.2 / 14.2; 9800 and 2318 17.8 / 16.6; 16,200
+    // and 4926 30.2 / 23.4.
+    if (!(learned ? halo_pays(p, 7680, 2) : halo_pays(p, 12800, 8))) return false;
     SmemBudget b;
     if (!b.take(static_cast<uint64_t>(p.lo) + p.mcap + p.hi, 4)) return false;
     if (learned) {
